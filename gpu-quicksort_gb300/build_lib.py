@@ -23,7 +23,7 @@ BUILD = os.path.join(HERE, "_build")
 INCLUDE = os.path.join(ROOT, "include")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
+NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++20", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
               "--expt-relaxed-constexpr", "-I" + CSRC, "-I" + INCLUDE]
 CU_SOURCES = ["gqs_sort_dispatch.cu", "gqs_capi.cu", "gqs_noalloc.cu", "gqs_batch.cu", "gqs_serve.cu",
               "gqs_merge.cu", "gqs_split.cu"]

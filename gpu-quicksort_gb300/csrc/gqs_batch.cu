@@ -27,6 +27,7 @@ GraphSort::~GraphSort() {
   drop_graphs();
   if (jobs_) cudaFree(jobs_);
   if (ring_) cudaFree(ring_);
+  if (split_) cudaFree(split_);
   if (q_) cudaFree(q_);
   if (hdr_dev_) cudaFree(hdr_dev_);
   if (q_host_) cudaFreeHost(q_host_);
@@ -58,12 +59,15 @@ gqs_status GraphSort::init(int device, int num_sms, size_t max_keys, size_t max_
   timeout_ms_ = timeout_ms ? timeout_ms : 4000;
   table_words_ = 1 + (pairs ? 2 * max_segs : max_segs + 1);
   // Job records and ring entries for the most demanding variant of any key type.
-  size_t cap = 0, ring = 0;
+  size_t cap = 0, ring = 0, split = 0;
+  const bool use_split = max_keys < (1ull << 31);
+  const size_t roots = use_split ? std::max(max_segs, max_keys / 4096 + 1) : max_segs;  // the split may leave so many ranges
+  for (int t = 0; t < 3 && use_split; ++t) split = std::max(split, split_scratch_bytes(t, max_keys, max_segs, false, num_sms));
   for (int t = 0; t < 3; ++t)
     for (int v = 0; v < variant_count(t); ++v) {
       const VariantInfo vi = variant_info(t, v);
-      cap = std::max(cap, job_capacity(vi, max_keys, max_segs));
-      ring = std::max(ring, ticket_ring(vi, max_keys, max_segs));
+      cap = std::max(cap, job_capacity(vi, max_keys, roots));
+      ring = std::max(ring, ticket_ring(vi, max_keys, roots));
     }
   if (cap >= (1ull << 32) || ring > (1ull << 31)) return GQS_ERR_INVALID;
   cudaError_t e;
@@ -71,6 +75,8 @@ gqs_status GraphSort::init(int device, int num_sms, size_t max_keys, size_t max_
   job_cap_ = cap;
   if ((e = cudaMalloc(&ring_, ring * sizeof(unsigned long long))) != cudaSuccess) return cuda_status(e);
   ring_len_ = ring;
+  if (split && (e = cudaMalloc(&split_, split)) != cudaSuccess) return cuda_status(e);
+  split_bytes_ = split;
   if ((e = cudaMalloc(&q_, sizeof(Queue))) != cudaSuccess) return cuda_status(e);
   if ((e = cudaMalloc(&hdr_dev_, table_words_ * sizeof(unsigned long long))) != cudaSuccess) return cuda_status(e);
   if ((e = cudaMallocHost(&q_host_, sizeof(Queue))) != cudaSuccess) return cuda_status(e);
@@ -149,9 +155,31 @@ gqs_status GraphSort::capture(int dtype, int variant) {
   };
   keep(cudaMemcpyAsync(hdr_dev_, hdr_host_, table_words_ * sizeof(unsigned long long), cudaMemcpyHostToDevice,
                        cap_stream_));
-  keep(cudaMemsetAsync(q_, 0, sizeof(Queue), cap_stream_));
+  if (!split_) keep(cudaMemsetAsync(q_, 0, sizeof(Queue), cap_stream_));
   keep(cudaMemsetAsync(ring_, 0, ring_len_ * sizeof(unsigned long long), cap_stream_));
-  if (first == cudaSuccess) keep(launch_sort(dtype, p));
+  if (split_) {
+    SplitArgs sa{};
+    sa.d = p.d;
+    sa.dn = p.dn;
+    sa.n = max_keys_;
+    sa.bound = p.n;
+    sa.offsets = p.offsets;
+    sa.nseg_dev = p.nseg_dev;
+    sa.nseg = max_segs_;
+    sa.pairs = p.pairs;
+    sa.scratch = split_;
+    sa.q = q_;
+    sa.sms = num_sms_;
+    sa.stream = cap_stream_;
+    SplitResult left{};
+    if (first == cudaSuccess) keep(split_launch(dtype, sa, &left));
+    p.offsets = left.table;
+    p.nseg_dev = left.count;
+    p.nseg = left.most;
+    p.pairs = 1;
+    p.from_dn = left.from_dn;
+  }
+  if (first == cudaSuccess && (!split_ || p.nseg)) keep(launch_sort(dtype, p));
   keep(cudaMemcpyAsync(q_host_, q_, sizeof(Queue), cudaMemcpyDeviceToHost, cap_stream_));
   cudaGraph_t g = nullptr;
   e = cudaStreamEndCapture(cap_stream_, &g);  // always ends the capture

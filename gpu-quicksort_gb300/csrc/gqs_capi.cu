@@ -129,6 +129,10 @@ struct gqs_ctx {
   cudaEvent_t ev_begin = nullptr, ev_end = nullptr, ev_done = nullptr;
   bool pending = false;
   bool pending_timed = false;
+  bool pending_copied = false;   // the status block is copied to q_host before ev_done
+  bool pending_rest = false;     // what the split may have left is not launched yet
+  gqs::LaunchParams rest{};
+  size_t rest_ring = 0;
   int pending_dtype = 0;
   int pending_variant = 0;
   int pending_grid = 0;
@@ -167,13 +171,39 @@ gqs_status grow(void** p, size_t* cap, size_t bytes) {
   return GQS_OK;
 }
 
+// The persistent kernel, after the ring it takes its work from is cleared.
+cudaError_t launch_quicksort(gqs_ctx* c, int dtype, const gqs::LaunchParams& p, size_t ring) {
+  // Only the part of the ring this sort can reach needs clearing.
+  cudaError_t e = cudaMemsetAsync(c->tmap, 0, ring * sizeof(unsigned long long), p.stream);
+  return e == cudaSuccess ? gqs::launch_sort(dtype, p) : e;
+}
+
+// Grows the split's scratch; no sort is using it.
+gqs_status grow_split(gqs_ctx* c, size_t bytes) {
+  const void* const old = c->split_buf;
+  const size_t had = c->split_bytes;
+  gqs_status st = grow(&c->split_buf, &c->split_bytes, bytes);
+  if (st == GQS_OK && (c->split_buf != old || c->split_bytes != had))
+    st = cuda_status(cudaMemset(c->split_buf, 0, gqs::split_clear_bytes()));
+  return st;
+}
+
 gqs_status wait_pending_locked(gqs_ctx* c) {
   if (!c->pending) return GQS_OK;
   cudaError_t e = cudaEventSynchronize(c->ev_done);
   if (e != cudaSuccess) return cuda_status(e);
-  e = cudaMemcpy(c->q_host, c->pending_acc ? c->q_acc : c->q, sizeof(gqs::Queue), cudaMemcpyDeviceToHost);
+  if (!c->pending_copied)
+    e = cudaMemcpy(c->q_host, c->pending_acc ? c->q_acc : c->q, sizeof(gqs::Queue), cudaMemcpyDeviceToHost);
+  c->pending_copied = false;
+  if (e == cudaSuccess && c->pending_rest && c->q_host->left && !c->q_host->error) {
+    e = launch_quicksort(c, c->pending_dtype, c->rest, c->rest_ring);
+    if (e == cudaSuccess) e = cudaEventRecord(c->ev_done, c->rest.stream);
+    if (e == cudaSuccess) e = cudaEventSynchronize(c->ev_done);
+    if (e == cudaSuccess) e = cudaMemcpy(c->q_host, c->q, sizeof(gqs::Queue), cudaMemcpyDeviceToHost);
+  }
   c->pending = false;
   c->pending_acc = false;
+  c->pending_rest = false;
   if (e != cudaSuccess) return cuda_status(e);
   gqs_stats s = gqs::stats_from_queue(*c->q_host, c->pending_dtype, c->pending_variant, c->pending_grid);
   if (c->pending_timed) {
@@ -203,19 +233,26 @@ gqs_status drain(gqs_ctx* c, gqs_status st) {
   return st;
 }
 
-// Validates, grows pools, and enqueues one sort on `stream`. Caller holds the lock.
+// Which sorts start with the split. A context with a fixed kernel variant keeps to it above 2^21 keys and below 2^15.
+bool use_split(const gqs_ctx* c, int dtype, size_t n, bool plain) {
+  if (!c->top_split || n >= (1ull << 31)) return false;
+  return !plain || c->auto_variant[dtype] || (n >= (1u << 15) && n <= (1u << 21));
+}
+
+// Validates, grows pools, and enqueues one sort on `stream`. Caller holds the lock. `waits`: the
+// caller waits for the sort next (wait_pending_locked), so the persistent kernel is launched only
+// then and only if the split has left it something.
 gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, const unsigned long long* offsets,
-                          size_t nseg, cudaStream_t stream, unsigned long long check_n = 0) {
+                          size_t nseg, cudaStream_t stream, unsigned long long check_n = 0, bool waits = false) {
   const size_t es = kElemSize[dtype];
   if (!d || (reinterpret_cast<uintptr_t>(d) % es) != 0) return GQS_ERR_INVALID;
   if (dn && (reinterpret_cast<uintptr_t>(dn) % es) != 0) return GQS_ERR_INVALID;
   if (n >= (1ull << 40) || nseg >= (1ull << 31)) return GQS_ERR_INVALID;
   const int v = c->auto_variant[dtype] ? gqs::tuned_variant(dtype, n, c->num_sms) : c->variant[dtype];
   const gqs::VariantInfo vi = gqs::variant_info(dtype, v);
-  // Small plain sorts start with a multi-way split whose buckets become the segments.
-  gqs::SplitPlan plan{};
-  const bool split = !offsets && !check_n && c->top_split && gqs::split_plan(dtype, n, vi.tile, c->num_sms, &plan);
-  const size_t segs = split ? plan.k : nseg;
+  const bool split = !check_n && use_split(c, dtype, n, offsets == nullptr);
+  const size_t split_bytes = split ? gqs::split_scratch_bytes(dtype, n, nseg, offsets == nullptr, c->num_sms) : 0;
+  const size_t segs = split ? std::max(nseg, n / 4096 + 1) : nseg;
   const size_t cap = job_capacity(vi, n, segs);
   const size_t ring = ticket_ring(vi, n, segs);
   if (cap >= (1ull << 32) || ring > (1ull << 31)) return GQS_ERR_INVALID;
@@ -227,7 +264,7 @@ gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, co
   const bool need_jobs = c->job_cap < cap;
   const bool need_dn = !dn && c->pool_dn_bytes < n * es;
   const bool need_ring = c->tmap_len < ring;
-  const bool need_split = split && c->split_bytes < gqs::split_scratch_bytes(plan);
+  const bool need_split = c->split_bytes < split_bytes;
   if (need_jobs || need_dn || need_ring || need_split) {
     st = wait_pending_locked(c);
     if (st != GQS_OK && st != GQS_ERR_TIMEOUT && st != GQS_ERR_CAPACITY && st != GQS_ERR_INTERNAL) return st;
@@ -253,7 +290,7 @@ gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, co
       if (st != GQS_OK) return st;
     }
     if (need_split) {
-      st = grow(&c->split_buf, &c->split_bytes, gqs::split_scratch_bytes(plan));
+      st = grow_split(c, split_bytes);
       if (st != GQS_OK) return st;
     }
   }
@@ -262,11 +299,7 @@ gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, co
     cudaError_t e = cudaStreamWaitEvent(stream, c->ev_done, 0);
     if (e != cudaSuccess) return cuda_status(e);
   }
-  cudaError_t e = cudaMemsetAsync(c->q, 0, sizeof(gqs::Queue), stream);
-  if (e != cudaSuccess) return cuda_status(e);
-  // Only the part of the ring this sort can reach needs clearing.
-  e = cudaMemsetAsync(c->tmap, 0, ring * sizeof(unsigned long long), stream);
-  if (e != cudaSuccess) return cuda_status(e);
+  cudaError_t e = cudaSuccess;
   gqs::LaunchParams p{};
   p.d = d;
   p.dn = dn;
@@ -288,18 +321,41 @@ gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, co
   if (split) {  // the timed interval starts with the split
     if (p.ev_begin && (e = cudaEventRecord(p.ev_begin, stream)) != cudaSuccess) return cuda_status(e);
     p.ev_begin = nullptr;
-    unsigned long long* table = nullptr;
-    e = gqs::split_launch(dtype, plan, d, dn, n, c->split_buf, &table, c->q, stream);
-    if (e != cudaSuccess) return cuda_status(e);
-    p.offsets = table;
-    p.nseg = plan.k;
-    p.from_dn = 1;
+    gqs::SplitArgs sa{};
+    sa.d = d;
+    sa.dn = dn;
+    sa.n = sa.bound = n;
+    sa.offsets = offsets;
+    sa.nseg = nseg;
+    sa.scratch = c->split_buf;
+    sa.q = c->q;
+    sa.sms = c->num_sms;
+    sa.stream = stream;
+    gqs::SplitResult left{};
+    if ((e = gqs::split_launch(dtype, sa, &left)) != cudaSuccess) return cuda_status(e);
+    p.offsets = left.table;
+    p.nseg_dev = left.count;
+    p.nseg = left.most;
+    p.pairs = 1;
+    p.from_dn = left.from_dn;
+    c->pending_rest = waits && left.most;
+    if ((waits || !left.most) && p.ev_end) e = cudaEventRecord(p.ev_end, stream);
+    if (c->pending_rest) {
+      c->rest = p;
+      c->rest_ring = ring;
+    }
+    if (e == cudaSuccess && !waits && left.most) e = launch_quicksort(c, dtype, p, ring);
+  } else {
+    c->pending_rest = false;
+    e = cudaMemsetAsync(c->q, 0, sizeof(gqs::Queue), stream);
+    if (e == cudaSuccess) e = launch_quicksort(c, dtype, p, ring);
   }
-  e = gqs::launch_sort(dtype, p);
-  if (e != cudaSuccess) return cuda_status(e);
-  e = cudaEventRecord(c->ev_done, stream);
+  if (e == cudaSuccess && waits)
+    e = cudaMemcpyAsync(c->q_host, c->q, sizeof(gqs::Queue), cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaEventRecord(c->ev_done, stream);
   if (e != cudaSuccess) return cuda_status(e);
   c->pending = true;
+  c->pending_copied = waits;
   c->pending_timed = c->cfg.timing != 0;
   c->pending_dtype = dtype;
   c->pending_variant = v;
@@ -313,7 +369,8 @@ gqs_status sort_dev(gqs_ctx* c, int dtype, void* d, void* scratch, size_t n, voi
   std::lock_guard<std::mutex> lk(c->mu);
   DeviceGuard dg(c->device);
   if (n <= 1) return d || n == 0 ? GQS_OK : GQS_ERR_INVALID;
-  gqs_status st = enqueue_locked(c, dtype, d, scratch, n, nullptr, 1, static_cast<cudaStream_t>(stream));
+  gqs_status st =
+      enqueue_locked(c, dtype, d, scratch, n, nullptr, 1, static_cast<cudaStream_t>(stream), 0, c->cfg.sync != 0);
   if (st != GQS_OK) return st;
   if (c->cfg.sync) return wait_pending_locked(c);
   return GQS_OK;
@@ -445,7 +502,7 @@ gqs_status sort_segments_dev(gqs_ctx* c, int dtype, void* keys, void* scratch, s
   if (nseg == 0) return GQS_OK;
   if (!offsets || !keys) return GQS_ERR_INVALID;
   gqs_status st = enqueue_locked(c, dtype, keys, scratch, n, reinterpret_cast<const unsigned long long*>(offsets),
-                                 nseg, static_cast<cudaStream_t>(stream));
+                                 nseg, static_cast<cudaStream_t>(stream), 0, c->cfg.sync != 0);
   if (st != GQS_OK) return st;
   if (c->cfg.sync) return wait_pending_locked(c);
   return GQS_OK;
@@ -698,14 +755,12 @@ gqs_status gqs_reserve(gqs_ctx* c, int dtype, size_t n, size_t nseg, int with_bu
     if (!c->blocks_per_sm[dtype][v]) return GQS_ERR_NO_DEVICE;
   }
   if (n >= (1ull << 40) || nseg >= (1ull << 31)) return GQS_ERR_INVALID;
-  // a plain sort of this size may start with the top split: its buckets are segments, and it
-  // has scratch of its own
-  gqs::SplitPlan plan{};
-  const bool split = nseg <= 1 && c->top_split && gqs::split_plan(dtype, n, vi.tile, c->num_sms, &plan);
-  if (split) {
-    nseg = plan.k;
-    gqs_status st = grow(&c->split_buf, &c->split_bytes, gqs::split_scratch_bytes(plan));
+  // the split has scratch of its own, and may leave ranges that become segments
+  const size_t nseg_in = nseg ? nseg : 1;
+  if (use_split(c, dtype, n, nseg <= 1)) {
+    gqs_status st = grow_split(c, gqs::split_scratch_bytes(dtype, n, nseg_in, nseg <= 1, c->num_sms));
     if (st != GQS_OK) return st;
+    nseg = std::max(nseg_in, n / 4096 + 1);
   }
   const size_t cap = job_capacity(vi, n, nseg ? nseg : 1);
   if (cap >= (1ull << 32) || ticket_ring(vi, n, nseg ? nseg : 1) > (1ull << 31)) return GQS_ERR_INVALID;
@@ -733,7 +788,7 @@ gqs_status gqs_reserve(gqs_ctx* c, int dtype, size_t n, size_t nseg, int with_bu
     st = grow(&c->pool_d, &c->pool_d_bytes, bytes);
     if (st != GQS_OK) return st;
     void* po = c->offs;
-    st = grow(&po, &c->offs_cap, ((nseg ? nseg : 1) + 1) * sizeof(uint64_t));
+    st = grow(&po, &c->offs_cap, (nseg_in + 1) * sizeof(uint64_t));
     c->offs = static_cast<unsigned long long*>(po);
     if (st != GQS_OK) return st;
   }

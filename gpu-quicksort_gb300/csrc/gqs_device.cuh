@@ -62,6 +62,7 @@ struct Queue {
   unsigned long long error_info;
   unsigned long long part_keys, local_keys, tiny_keys, fill_keys, chunks;
   uint32_t part_jobs, local_jobs, fill_jobs, max_depth;
+  uint32_t left, pad;        // ranges the split left to the persistent kernel
   // Cycles of each CTA's consumer leader thread, summed over CTAs: [1] on-chip sorts (tile wait,
   // sort, write-out), [2] queued pivot-run fills, [3] the whole consumer loop; the rest of [3] is
   // partition chunks, pipeline drains and waits for work ([0] is unused: a clock read per chunk
@@ -1905,6 +1906,9 @@ __global__ void __launch_bounds__(C::NT, min_blocks_per_sm<C>()) persistent_kern
   }
   __syncthreads();
   pdl_wait();  // the seed kernel's jobs and tickets are visible from here on
+  // No job was published and every key is placed (the split left nothing, or the segments were tiny): with no job nobody
+  // changes these, so every thread of every CTA sees the same. An empty launch takes 4 us so instead of 9.
+  if (ld_relaxed(&a.q->alloc) == 0ull && ld_relaxed(&a.q->total) == ld_relaxed(&a.q->done)) return;
 #ifdef GQS_PROFILE
   if (tid == 0) atomicCAS(&a.q->lvl_start, 0ull, (unsigned long long)global_timer_ns());
 #endif

@@ -101,19 +101,33 @@ cudaError_t merge_tiles(int dtype, const void* a, size_t na, const void* b, size
 cudaError_t merge_runs(int dtype, const void* a, size_t na, const void* b, size_t nb, void* out,
                        unsigned long long* splits, cudaStream_t s);
 
-// Top split of a plain sort of n keys (defined in gqs_split.cu): picks K - 1 splitters from
-// sorted samples of d, counts every key's bucket per CTA, scans the counts into bucket offsets
-// (segs, K + 1 entries) and scatters the keys into dn bucket by bucket. The buckets are then
-// sorted as segments whose keys are in dn. `scratch` holds split_scratch_bytes(dtype, n) bytes.
-struct SplitPlan {
-  uint32_t k;      // buckets (a power of two, 2 .. 1024)
-  uint32_t lg;     // log2 k
-  uint32_t ctas;   // CTAs of the count and scatter kernels
-  uint32_t samples;
+// The split sort (defined in gqs_split.cu): splits the array (or every segment) into many ranges by
+// sampled pivots and sorts the ranges on chip. What it leaves (ranges too long for that) is a
+// table of (start, end) pairs for the persistent kernel, most often empty; Queue::left says how many.
+// Clears the status block first.
+struct SplitArgs {
+  void* d;
+  void* dn;
+  size_t n;                            // keys in all, fewer than 2^31
+  unsigned long long bound;            // every key index is below it (n when offsets is null)
+  const unsigned long long* offsets;   // as in LaunchParams; null: one segment [0, n)
+  const unsigned long long* nseg_dev;
+  size_t nseg;
+  uint32_t pairs;
+  void* scratch;                       // split_scratch_bytes(dtype, n, nseg, offsets == null)
+  Queue* q;
+  int sms;
+  cudaStream_t stream;
 };
-bool split_plan(int dtype, size_t n, int tile, int sms, SplitPlan* plan);
-size_t split_scratch_bytes(const SplitPlan& plan);
-cudaError_t split_launch(int dtype, const SplitPlan& plan, const void* d, void* dn, size_t n, void* scratch,
-                         unsigned long long** segs, Queue* q, cudaStream_t s);
+struct SplitResult {
+  const unsigned long long* table;  // (start, end) of every range left
+  const unsigned long long* count;  // how many, on the device
+  uint32_t most;                    // at most this many (0: nothing can be left)
+  uint32_t from_dn;                 // 1: their keys are in dn
+};
+size_t split_scratch_bytes(int dtype, size_t n, size_t nseg, bool plain, int sms);
+size_t split_clear_bytes();  // the scratch's first bytes, to be zeroed once when it is allocated
+cudaError_t split_launch(int dtype, const SplitArgs& a, SplitResult* out);
+constexpr size_t kDtypeBytes(int dtype) { return dtype == DT_U32 || dtype == DT_F32 ? 4 : 8; }
 
 }  // namespace gqs

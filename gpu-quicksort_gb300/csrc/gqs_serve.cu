@@ -449,14 +449,7 @@ gqs_status gqs_srv_create(int device, const gqs_server_config* cfg, gqs_server**
       if (!c.per_request) {
         l->gs = std::make_unique<gqs::GraphSort>();
         st = l->gs->init(device, num_sms, c.batch_keys, c.batch_segments, true, c.timeout_ms);
-        size_t cap = 0, ring = 0;
-        for (int t = 0; t < 3; ++t)
-          for (int v = 0; v < gqs::variant_count(t); ++v) {
-            const gqs::VariantInfo vi = gqs::variant_info(t, v);
-            cap = std::max(cap, gqs::job_capacity(vi, c.batch_keys, c.batch_segments));
-            ring = std::max(ring, gqs::ticket_ring(vi, c.batch_keys, c.batch_segments));
-          }
-        lane_bytes += cap * sizeof(gqs::Job) + ring * 8;
+        lane_bytes += l->gs->record_bytes();
       }
       s->lanes.push_back(std::move(l));
     }
@@ -469,7 +462,7 @@ gqs_status gqs_srv_create(int device, const gqs_server_config* cfg, gqs_server**
       st = gqs_create(&s->plain, device, &pc);
       if (st != GQS_OK) break;
       for (int t = 0; t < 3; ++t) {
-        st = gqs_set_variant(s->plain, t, s->variant[t]);
+        if (c.variant[t] >= 0) st = gqs_set_variant(s->plain, t, s->variant[t]);
         if (st == GQS_OK) st = gqs_reserve(s->plain, t, c.batch_keys, 1, 0);
         if (st != GQS_OK) break;
       }

@@ -1,26 +1,29 @@
-// Top split of a small plain sort: one multi-way partition of the whole array into buckets
-// that the persistent kernel then sorts as segments (most of them as single on-chip tiles).
+// The split sort: quicksort's partition with hundreds of pivots at once, and an on-chip sort of the
+// ranges it leaves.
 //
-// Below a few million keys a binary partition level is bound by latency, not bandwidth: each
-// level waits for its jobs' last chunks, the completer's pivot sampling and the publication of
-// the children (about 11 us a level on a GB300), and 2^20 keys need seven levels before every
-// range fits one on-chip tile. The split replaces those levels with four short kernels over an
-// array that stays in L2:
-//   split_pick     one CTA: sorts 8 samples per bucket (runs of 256 by warp networks, then
-//                  merged pairwise by merge path) and keeps every 8th as a splitter, stored
-//                  as a breadth-first search tree (the on-chip split's layout and bucket rule:
-//                  bucket b holds splitter[b-1] < key <= splitter[b]);
-//   split_count    every CTA walks the tree for each key of its slice, counts per bucket in
-//                  shared memory and adds its counts to the bucket totals;
-//   split_starts   one CTA: exclusive scan of the bucket totals into the segment table and the
-//                  scatter cursors;
-//   split_scatter  every CTA walks the tree again, reserves its share of each bucket with one
-//                  atomic and appends each key to its bucket in dn.
-// The split is the reference's partition generalised from one pivot to k - 1 (the sample split
-// the on-chip sort already uses for a tile, applied once to the whole array); its pass is
-// counted in the sort's partition keys.
+// A binary partition level reads and writes every key to gain one bit of order, and a sort of 2^28
+// keys needs about fifteen before its ranges fit on chip. Here one level puts every key into one
+// of up to 1024 ranges, so two levels reach ranges of a few thousand keys at 2^28, and one level
+// reaches them below four million keys:
+//   split_map      one CTA a segment: a map of a key to its range, from a sample of the segment
+//   split_count    every key's range, counted
+//   split_starts   where every range starts; ranges still too long become segments of the next level
+//   split_scatter  every key to its range (d -> dn at the first level, dn -> d at the second)
+//   local_sort     every range sorted in shared memory, into d
+// Plain sorts of at most kSmallMax keys take two kernels instead: split_small (every CTA makes the
+// map for itself, then scatters into ranges with room for kLocal keys each, so that nothing is
+// counted first) and local_sort over those ranges.
+// The order of keys inside a range does not matter to the next step, so a key's place in it
+// is the old value of a counter (one shared-memory atomic), not a stable rank.
+//
+// What cannot be sorted so (a range that stays longer than the on-chip sort takes, because the map's
+// sample missed its keys) is listed for the persistent kernel's quicksort; Queue::left counts it.
+//
+// The reference's counterparts: gqsort_kernel's partition (GPU-Quicksort_OpenCL_1.2/
+// QuicksortKernels.cl:102-240) generalised from one pivot, and lqsort_kernel (267-421).
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdint>
 
 #include "gqs_device.cuh"
@@ -29,320 +32,1828 @@
 namespace gqs {
 namespace {
 
-constexpr int kThreads = 512;
-constexpr int kRun = 256;            // samples per warp-sorted run (8 per lane)
-constexpr uint32_t kMaxK = 1024;     // buckets
-constexpr uint32_t kMaxSamples = 4096;
-constexpr uint32_t kOversample = 8;  // samples per bucket
-constexpr uint32_t kMaxSlice = 16384;  // keys of one CTA's slice in the scatter (labels in shared memory)
-
 template <class T>
 using BOf = typename KeyOps<T>::B;
 
-// Dynamic shared memory of split_pick: two sample buffers.
-extern __shared__ __align__(16) unsigned char split_dyn[];
-
-template <class T>
-__global__ void __launch_bounds__(kThreads) split_pick(const BOf<T>* __restrict__ d, unsigned long long n, uint32_t k,
-                                                        uint32_t lg, uint32_t ns, BOf<T>* __restrict__ tree,
-                                                        uint32_t* __restrict__ total, Queue* q) {
-  using B = BOf<T>;
-  B* src = reinterpret_cast<B*>(split_dyn);
-  B* dst = src + kMaxSamples;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  pdl_trigger();  // split_count may launch now; it waits for this grid before reading the tree
-  for (uint32_t i = tid; i < k; i += kThreads) total[i] = 0u;
-#ifdef GQS_PROFILE
-  if (tid == 0) atomicCAS(&q->lvl_start, 0ull, (unsigned long long)global_timer_ns());  // per-level times start here
-#else
-  (void)q;
+#ifndef SP_KPT32
+#define SP_KPT32 16
 #endif
-  const uint32_t nrun = ns / kRun;
-  if ((uint32_t)warp < nrun) {
-    B v[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const unsigned long long i = (unsigned long long)warp * kRun + (unsigned long long)(r * 32 + lane);
-      v[r] = KeyOps<T>::key(d[(i * n) / ns]);
-    }
-    warp_bitonic_n<8, 1, B>(v);  // element lane * 8 + r of the run
-#pragma unroll
-    for (int r = 0; r < 8; ++r) src[warp * kRun + lane * 8 + r] = v[r];
-  }
-  __syncthreads();
-  // Merge the sorted runs pairwise until one run remains: each thread writes `per` consecutive
-  // outputs of one pair, starting where merge path puts its first output (the number of keys
-  // the first run contributes before it, by binary search on the diagonal).
-  const uint32_t per = ns / kThreads;  // ns is 256 << j; with ns >= 512, per divides every pair
-  for (uint32_t len = kRun; len < ns; len <<= 1) {
-    if (per > 0) {
-      const uint32_t o0 = (uint32_t)tid * per, base = o0 / (2u * len) * (2u * len), dg = o0 - base;
-      const B* x = src + base;
-      const B* y = x + len;
-      uint32_t lo = dg > len ? dg - len : 0u, hi = dg < len ? dg : len;
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (x[mid] <= y[dg - 1u - mid]) lo = mid + 1u;
-        else hi = mid;
-      }
-      uint32_t i = lo, j = dg - lo;
-      for (uint32_t t = 0; t < per; ++t) {
-        const bool from_x = j >= len || (i < len && x[i] <= y[j]);
-        dst[o0 + t] = from_x ? x[i++] : y[j++];
-      }
-    }
-    __syncthreads();
-    B* const tmp = src;
-    src = dst;
-    dst = tmp;
-  }
-  // splitter q1 - 1 is the sample of rank q1 * step - 1
-  const uint32_t step = ns / k;
-  for (uint32_t q1 = (uint32_t)tid + 1u; q1 < k; q1 += kThreads) {
-    const uint32_t tz = (uint32_t)__ffs(q1) - 1u;
-    tree[(1u << (lg - 1u - tz)) + (q1 >> (tz + 1u))] = src[q1 * step - 1u];
-  }
-}
+#ifndef SP_MINB
+#define SP_MINB 2
+#endif
+#ifndef LS_NT32
+#define LS_NT32 256
+#endif
+#ifndef LS_MINB32
+#define LS_MINB32 3
+#endif
+#ifndef LS_LT32
+#define LS_LT32 8192
+#endif
+#ifndef LS_NT64
+#define LS_NT64 256
+#endif
+#ifndef LS_MINB64
+#define LS_MINB64 3
+#endif
+#ifndef LS_LT64
+#define LS_LT64 4096
+#endif
+#ifndef SP_OVER
+#define SP_OVER 32
+#endif
+constexpr int kThreads = 512;
+constexpr uint32_t kMaxBins = 1024;             // ranges one segment is split into (bin_room: the map may make more)
+constexpr uint32_t kBinSlots = 2564;            // bin_room(kMaxBins)
+constexpr uint32_t kMaxCells = 4096;
+constexpr uint32_t kMaxParts = 256;             // cells divided further
+constexpr uint32_t kMaxSub = 2048;              // cells that those are divided into
+constexpr uint32_t kPartSub = 128;              // and at most so many for one
+constexpr uint32_t kShortBin = 9;               // longest bin that the networks of the on-chip sort put in order
+constexpr uint32_t kWarpBin = 256;              // longer ones of unequal keys are sorted by a warp each, beyond this by the CTA
+constexpr int kCandidates = 4;
+constexpr uint32_t kCopyChunk = 32768;          // keys of one record of a range of equal keys
+constexpr uint32_t kSmallOver = 10;             // samples a range of a small sort (its ranges have room for three times their mean)
 
+template <class B>
+struct Sizes {
+  static constexpr uint32_t kLocal = sizeof(B) == 8 ? LS_LT64 : LS_LT32;  // keys one CTA sorts on chip
+  static constexpr uint32_t kSortThreads = sizeof(B) == 8 ? LS_NT64 : LS_NT32, kSortCtas = sizeof(B) == 8 ? LS_MINB64 : LS_MINB32;
+  static constexpr uint32_t kTarget = kLocal / 16 * 7;      // mean keys of a range
+  static constexpr int kTileRows = SP_KPT32 * 4 / (int)sizeof(B);
+  static constexpr uint32_t kTile = kThreads * kTileRows;
+  static constexpr int kLocalRows = (int)(kLocal / kSortThreads);
+  static constexpr uint32_t kTiny = sizeof(B) == 8 ? 128 : 256;
+  // keys of a sample: at the first level of a plain sort (one CTA), at other levels, and in a small sort (two CTAs an SM)
+  static constexpr uint32_t kMaxSample = sizeof(B) == 8 ? 16384 : 24576, kMaxSample2 = sizeof(B) == 8 ? 8192 : 12288;
+  static constexpr uint32_t kSmallSample = sizeof(B) == 8 ? 3328 : 5120;
+  static constexpr size_t kSmallMax = sizeof(B) == 8 ? 1u << 19 : 1u << 21;
+};
 template <class T>
-__device__ __forceinline__ uint32_t bucket_of(const BOf<T>* t, uint32_t lg, BOf<T> key) {
-  uint32_t b = 1u;
-  for (uint32_t l = 0; l < lg; ++l) b = 2u * b + (t[b] < key ? 1u : 0u);
-  return b;
-}
-
-// Buckets (0 .. k-1) of kBatch keys per thread at once: keys lo + tid + j * kThreads of
-// [lo, hi); all loads are issued before the tree walks, which then run interleaved. Keys past
-// hi get bucket kNone.
-constexpr int kBatch = 8;
-constexpr uint32_t kNone = 0xffffffffu;
+using EngineCfg = Cfg<T, 16, sizeof(BOf<T>) == 8 ? 6144 : 12288, sizeof(BOf<T>) == 8 ? 4096 : 8192, 3, sizeof(BOf<T>) == 8 ? 4 : 8>;
 template <class T>
-__device__ __forceinline__ void buckets_of(const BOf<T>* __restrict__ d, unsigned long long i0, unsigned long long hi,
-                                           const BOf<T>* t, uint32_t k, uint32_t lg, uint32_t (&b)[kBatch],
-                                           BOf<T> (&raw)[kBatch]) {
-  BOf<T> key[kBatch];
-#pragma unroll
-  for (int j = 0; j < kBatch; ++j) {
-    const unsigned long long i = i0 + (unsigned long long)j * kThreads;
-    raw[j] = i < hi ? d[i] : BOf<T>(0);
-    key[j] = KeyOps<T>::key(raw[j]);
-    b[j] = 1u;
+constexpr bool kFloating = !KeyOps<T>::kIdentity;
+
+constexpr uint32_t kEqual = 1u << 30, kBinMask = 0xffffu;  // in a map's table: all keys of the range are equal; the range
+
+// A segment being split: its keys, and the map of a key to its range.
+struct SegRec {
+  unsigned long long start;
+  unsigned long long lo, span;  // keys are clamped to [lo, lo + span]
+  uint32_t len, k, cells;       // cells allocated (a power of two)
+  uint32_t bin0, cell0, tile0;  // its counters, map cells and tiles
+  uint32_t sh, bins, used;      // entries of the table; cell of a key: (key - lo) >> sh, or by value:
+  float flo, scale;             // (key - flo) * scale, in 4096ths of a cell
+  uint32_t top;                 // greatest value of that
+  uint32_t kind;                // BY_VALUE, PARTS, and how many Part records there are
+};
+enum : uint32_t { BY_VALUE = 1u << 31, PARTS = 1u << 30, PART_COUNT = PARTS - 1u };
+// A cell with more than the sample of one range, divided further: equal steps between its least and greatest sampled key, or
+// (mult 0) the keys below, equal to and above one value that makes up nearly all of them.
+template <class B>
+struct Part {
+  B lo, span;
+  uint32_t right, left, mult;  // the span shifted to just below 2^32, times mult / 2^32
+  uint32_t sub;                // its cells in the table start here
+  __device__ __forceinline__ uint32_t of(B key) const {
+    if (!mult) return sub + (key >= lo ? 1u : 0u) + (key > lo ? 1u : 0u);
+    B y = (key < lo ? lo : key) - lo;
+    y = y < span ? y : span;
+    return sub + __umulhi((uint32_t)(y >> right) << left, mult);
   }
-  for (uint32_t l = 0; l < lg; ++l) {
-#pragma unroll
-    for (int j = 0; j < kBatch; ++j) b[j] = 2u * b[j] + (t[b[j]] < key[j] ? 1u : 0u);
-  }
-#pragma unroll
-  for (int j = 0; j < kBatch; ++j) b[j] = i0 + (unsigned long long)j * kThreads < hi ? b[j] - k : kNone;
+};
+enum : uint32_t { IN_DN = 1, EQUAL = 2 };
+struct Bucket {
+  unsigned long long start;
+  uint32_t len, flags;
+  unsigned long long value;  // EQUAL: all keys are this
+};
+struct alignas(256) Ctl {
+  unsigned long long alloc[2];  // (segments << 32) | tiles, per level
+  unsigned long long leftovers;
+  uint32_t bins[2], cells[2];
+  uint32_t buckets;
+};
+
+// The tables of one level.
+struct Level {
+  SegRec* seg;
+  uint32_t* bin;   // keys per range, then the next output position in it (from the segment's start)
+  unsigned long long* value;  // kEqual ranges: the keys, as the map orders them
+  uint32_t* eq;               // 1: a kEqual range
+  uint32_t* cell;
+  void* part;      // the records of the cells with a map of their own (part_room(k) for a segment, at bin0 / 4)
+  uint32_t segs, bins, cells;  // how many there is room for
+  uint32_t index;
+};
+struct Tables {
+  Ctl* ctl;
+  Bucket* bucket;
+  unsigned long long* left;  // (start, end) of the ranges left to the quicksort
+  uint32_t buckets;          // records there is room for
+  uint32_t tile_keys;
+};
+// The state of a small plain sort. The cursors and the count of finished CTAs are zero between sorts: the last CTA of
+// local_small leaves them so.
+struct Small {
+  uint32_t cursor[kBinSlots];              // next place in every range
+  uint32_t done;                           // CTAs of local_small that have finished
+  uint32_t bins;
+  unsigned long long left;                 // 1: all of the sort is left to the persistent kernel
+  unsigned long long table[2];             // (then: [0, n))
+  uint32_t eq[kBinSlots];                  // 1: all keys of the range are equal (the cursor counts them, none is moved)
+  unsigned long long value[kBinSlots];     // to this (as the map orders keys)
+};
+
+__device__ __forceinline__ uint32_t ceil_log2(uint32_t v) { return v <= 1u ? 0u : 32u - (uint32_t)__clz(v - 1u); }
+
+// Counters of a segment split k ways: at most k + 1 ranges, and two for each single value with the sample of 1.5 ranges.
+__device__ __host__ __forceinline__ uint32_t bin_room(uint32_t k) { return 2u * k + k / 2u + 4u; }
+__device__ __host__ __forceinline__ uint32_t part_room(uint32_t k) { return k / 2u + 1u < kMaxParts ? k / 2u + 1u : kMaxParts; }
+__device__ __host__ __forceinline__ uint32_t sub_room(uint32_t k) { return 8u * k + 32u < kMaxSub ? 8u * k + 32u : kMaxSub; }
+__device__ __forceinline__ uint32_t cell_count(uint32_t k) {
+  const uint32_t l = ceil_log2(4u * k);
+  return 1u << (l < 8u ? 8u : l > 12u ? 12u : l);
 }
 
-// CTA c's slice of the keys: [c * n / ctas, (c + 1) * n / ctas).
-__device__ __forceinline__ void slice_of(unsigned long long n, uint32_t ctas, unsigned long long& lo,
-                                         unsigned long long& hi) {
-  lo = n * blockIdx.x / ctas;
-  hi = n * (blockIdx.x + 1ull) / ctas;
+// False: no room (only segments that overlap, which no valid table has, can need more than there is).
+__device__ __forceinline__ bool add_segment(const Tables& t, const Level& v, unsigned long long start, uint32_t len, uint32_t k) {
+  SegRec r{};
+  r.start = start;
+  r.len = len;
+  r.k = k;
+  r.cells = cell_count(k) + sub_room(k);
+  r.bin0 = atomicAdd(&t.ctl->bins[v.index], bin_room(k));
+  r.cell0 = atomicAdd(&t.ctl->cells[v.index], r.cells);
+  const uint32_t tiles = (len + t.tile_keys - 1u) / t.tile_keys;
+  const unsigned long long old = atomicAdd(&t.ctl->alloc[v.index], (1ull << 32) | (unsigned long long)tiles);
+  r.tile0 = (uint32_t)old;
+  const uint32_t at = (uint32_t)(old >> 32);
+  if (at >= v.segs || r.bin0 + bin_room(k) > v.bins || r.cell0 + r.cells > v.cells) return false;
+  v.seg[at] = r;
+  return true;
 }
 
+// Ranges for `len` keys: enough for a mean of kTarget keys, or with more than kMaxBins needed and a
+// second level to come, the square root.
+template <class B>
+__device__ __host__ __forceinline__ uint32_t range_count(uint32_t len, bool more_levels) {
+  const uint32_t want = (len + Sizes<B>::kTarget - 1u) / Sizes<B>::kTarget;
+  if (want <= 2u) return 2u;
+  if (want <= kMaxBins) return want;
+  if (!more_levels) return kMaxBins;
+  const uint32_t r = (uint32_t)ceilf(sqrtf((float)want));
+  return r < kMaxBins ? r : kMaxBins;
+}
+
+// Zeroes `bytes` (a multiple of 4) at p with the calling CTA.
+__device__ __forceinline__ void clear(void* p, size_t bytes) {
+  for (uint32_t i = threadIdx.x; i < bytes / 4; i += blockDim.x) static_cast<volatile uint32_t*>(p)[i] = 0u;
+}
+
+// ---- segments: short ones are sorted or listed, long ones are to be split -------------------
 template <class T>
-__global__ void __launch_bounds__(kThreads) split_count(const BOf<T>* __restrict__ d, unsigned long long n, uint32_t k,
-                                                         uint32_t lg, const BOf<T>* __restrict__ tree,
-                                                         uint32_t* __restrict__ total) {
+__global__ void __launch_bounds__(256) split_plan_segments(SortArgs<T> a, Tables t, Level v, const unsigned long long* offsets,
+                                                           const unsigned long long* nseg_dev, uint32_t nseg,
+                                                           unsigned long long n, uint32_t pairs, uint32_t levels) {
   using B = BOf<T>;
-  __shared__ B t[kMaxK];
-  __shared__ uint32_t cnt[kMaxK];
+  __shared__ unsigned long long placed_sum;
+  const uint32_t seg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   pdl_wait();
   pdl_trigger();
-  for (uint32_t i = threadIdx.x; i < k; i += kThreads) {
-    t[i] = tree[i];
-    cnt[i] = 0u;
+  if (nseg_dev) {
+    const unsigned long long m = *nseg_dev;
+    if (m > nseg) {
+      if (seg == 0 && lane == 0) set_error(a.q, ST_INVALID, m);
+      return;
+    }
+    nseg = (uint32_t)m;
+  }
+  if (threadIdx.x == 0) placed_sum = 0ull;
+  __syncthreads();
+  if (seg < nseg) {
+    const unsigned long long s = offsets[pairs ? 2ull * seg : seg], e = offsets[pairs ? 2ull * seg + 1 : seg + 1];
+    if (s > e || e > n) {  // malformed segment table
+      if (lane == 0) set_error(a.q, ST_INVALID, seg);
+    } else if (e > s) {
+      const unsigned long long m = e - s;
+      if (m <= Sizes<B>::kTiny) {
+        unsigned long long tiny = 0;
+        const unsigned long long placed = place_small<EngineCfg<T>>(a, 1u, s, m, tiny);
+        if (lane == 0) atomicAdd(&placed_sum, placed);
+      } else if (lane == 0) {
+        bool room = m < (1ull << 31);
+        if (m <= Sizes<B>::kLocal) {
+          const uint32_t at = atomicAdd(&t.ctl->buckets, 1u);
+          room = at < t.buckets;
+          if (room) t.bucket[at] = Bucket{s, (uint32_t)m, 0u, 0ull};
+        } else if (room) {
+          room = add_segment(t, v, s, (uint32_t)m, range_count<B>((uint32_t)m, levels > 1u));
+        }
+        if (!room) set_error(a.q, ST_CAPACITY, seg);
+      }
+    }
   }
   __syncthreads();
-  unsigned long long lo, hi;
-  slice_of(n, gridDim.x, lo, hi);
-  for (unsigned long long i0 = lo + threadIdx.x; i0 < hi; i0 += (unsigned long long)kBatch * kThreads) {
-    uint32_t b[kBatch];
-    B raw[kBatch];
-    buckets_of<T>(d, i0, hi, t, k, lg, b, raw);
-#pragma unroll
-    for (int j = 0; j < kBatch; ++j)
-      if (b[j] != kNone) atomicAdd(&cnt[b[j]], 1u);
+  if (threadIdx.x == 0 && placed_sum) {
+    atomicAdd(&a.q->total, placed_sum);
+    atomicAdd(&a.q->done, placed_sum);
+    atomicAdd(&a.q->tiny_keys, placed_sum);
   }
-  __syncthreads();
-  for (uint32_t b = threadIdx.x; b < k; b += kThreads)
-    if (cnt[b]) atomicAdd(&total[b], cnt[b]);
 }
 
-// One CTA of kMaxK threads: bucket starts from the bucket totals (exclusive scan); they become
-// the segment table (segs[k] = n) and the scatter cursors.
-__global__ void __launch_bounds__(kMaxK) split_starts(const uint32_t* __restrict__ total, uint32_t k,
-                                                      unsigned long long n, uint32_t* __restrict__ cursor,
-                                                      unsigned long long* __restrict__ segs, Queue* q) {
-  __shared__ uint32_t wsum[32];
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  pdl_wait();
-  pdl_trigger();
-  const uint32_t c = tid < k ? total[tid] : 0u;
-  uint32_t inc = c;
+// ---- the map of a segment, from a sample of its keys --------------------------------------------
+__device__ __forceinline__ int bits_of(uint32_t v) { return 32 - __clz((int)v); }
+__device__ __forceinline__ int bits_of(uint64_t v) { return 64 - __clzll((long long)v); }
+
+// A key of a floating type as a float (a double rounded towards zero, beyond the float range cut
+// off), in the keys' order.
+template <class T>
+__device__ __forceinline__ float as_float(BOf<T> key) {
+  if constexpr (sizeof(BOf<T>) == 4) {
+    return __uint_as_float((uint32_t)KeyOps<T>::raw(key));
+  } else {
+    const uint64_t r = KeyOps<T>::raw(key);
+    const uint32_t hi = (uint32_t)(r >> 32), mag = hi & 0x7fffffffu;
+    uint32_t f = __funnelshift_l((uint32_t)r, mag, 3) - (896u << 23);  // the exponent's bias from 1023 to 127
+    f = mag < 0x38100000u ? 0u : mag >= 0x47f00000u ? 0x7f7fffffu : f;
+    return __uint_as_float(f | (hi & 0x80000000u));
+  }
+}
+// Both ends and their distance are ordinary floats.
+__device__ __forceinline__ bool finite_span(float a, float b, float w) {
+  return w > 0.f && w < 3e38f && fabsf(a) < 3e38f && fabsf(b) < 3e38f;
+}
+
+// The range of a key: a table's entry for its cell, or (a cell with many samples) for the part of the cell that it is in, and so
+// on. Cells are equal steps of the integer that orders the keys, or (floating types, where that spreads the sample more evenly)
+// of their value. Every step of it keeps the order of the keys, and every kernel computes the same. VALUE and PARTS_ say what
+// the segment's kind asks for: a map of integer cells without parts is one table read and a few integer instructions a key.
+template <class T>
+struct KeyMap {
+  using B = BOf<T>;
+  B lo, span;
+  uint32_t sh, used, top, kind;
+  float flo, scale;
+  __device__ __forceinline__ void load(const SegRec& r) {
+    lo = (B)r.lo;
+    span = (B)r.span;
+    sh = r.sh;
+    used = r.used;
+    top = r.top;
+    kind = r.kind;
+    flo = r.flo;
+    scale = r.scale;
+  }
+  __device__ __forceinline__ B offset(B key) const {
+    const B x = (key < lo ? lo : key) - lo;
+    return x < span ? x : span;
+  }
+  template <bool VALUE>
+  __device__ __forceinline__ uint32_t cell(B key) const {
+    if constexpr (VALUE) {
+      const uint32_t u = __float2uint_rz(__fmul_rn(__fsub_rn(as_float<T>(lo + offset(key)), flo), scale));
+      return u < top ? u : top;
+    } else {
+      return (uint32_t)(offset(key) >> sh);
+    }
+  }
+  template <bool VALUE, bool PARTS_>
+  __device__ __forceinline__ uint32_t bin(B key, const uint32_t* tab, const Part<B>* part) const {
+    uint32_t e = tab[cell<VALUE>(key)];
+    if constexpr (PARTS_)
+      while (e >> 31) e = tab[part[e & 0x7fffffffu].of(key)];
+    return e;
+  }
+};
+// Calls f.template operator()<VALUE, PARTS_>() with what `kind` says.
+template <class T, class F>
+__device__ __forceinline__ void by_kind(uint32_t kind, F&& f) {
+  if (kFloating<T> && (kind & BY_VALUE)) {
+    if (kind & PARTS) f.template operator()<kFloating<T>, true>();
+    else f.template operator()<kFloating<T>, false>();
+  } else {
+    if (kind & PARTS) f.template operator()<false, true>();
+    else f.template operator()<false, false>();
+  }
+}
+
+template <class B>
+__device__ __forceinline__ B warp_min(B v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const B w = __shfl_xor_sync(0xffffffffu, v, o);
+    v = w < v ? w : v;
+  }
+  return v;
+}
+template <>
+__device__ __forceinline__ uint32_t warp_min<uint32_t>(uint32_t v) { return __reduce_min_sync(0xffffffffu, v); }
+template <class B>
+__device__ __forceinline__ B warp_max(B v) { return ~warp_min<B>(~v); }
+
+// Exclusive scan over the CTA of one value a thread; returns the sum through `total`.
+template <int NT>
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* wsum, uint32_t& total) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t inc = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-    if ((int)lane >= o) inc += v;
+    const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+    if ((int)lane >= o) inc += u;
   }
   if (lane == 31) wsum[warp] = inc;
   __syncthreads();
-  if (warp == 0) {
-    const uint32_t w = wsum[lane];
-    uint32_t wi = w;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xffffffffu, wi, o);
-      if ((int)lane >= o) wi += v;
-    }
-    wsum[lane] = wi - w;
-  }
+  const uint32_t w = lane < NT / 32 ? wsum[lane] : 0u;
+  total = __reduce_add_sync(0xffffffffu, w);
+  const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u);
   __syncthreads();
-  if (tid < k) {
-    const uint32_t start = wsum[warp] + inc - c;
-    cursor[tid] = start;
-    segs[tid] = start;
-  }
-  if (tid == 0) {
-    segs[k] = n;
-    atomicAdd(&q->part_keys, n);  // the split is one partition job and one pass over every key
-    atomicAdd(&q->part_jobs, 1u);
-#ifdef GQS_PROFILE
-    level_note(q, 0, 0, n);  // and the depth-0 job of the profiling library's per-level rows
-#endif
-  }
+  return inc - v + before;
 }
 
-// Every CTA labels the keys of its slice (labels kept in shared memory), reserves its share of
-// every bucket with one global atomic per bucket, and appends each key to its bucket in dn. The
-// order of the CTAs' shares inside a bucket does not matter: the bucket is sorted afterwards.
-template <class T>
-__global__ void __launch_bounds__(kThreads) split_scatter(const BOf<T>* __restrict__ d, BOf<T>* __restrict__ dn,
-                                                           unsigned long long n, uint32_t k, uint32_t lg,
-                                                           const BOf<T>* __restrict__ tree,
-                                                           uint32_t* __restrict__ cursor) {
+template <class B>
+struct MapSmem {
+  uint32_t tab[kMaxCells + kMaxSub];  // samples per cell, then the map's table
+  Part<B> part[kMaxParts];
+  uint16_t node[kMaxCells + kMaxSub];  // the part that a cell is divided into (kNone: it is not)
+  uint32_t weight[kMaxParts];          // two for each single value in the part
+  uint32_t entry[kMaxParts], owner[kMaxParts];  // the part's own cell, and the part that that is in
+  uint32_t before[kMaxParts], extra[kMaxParts];  // samples, and weights, in front of it
+  unsigned long long least[kMaxParts], greatest[kMaxParts];
+  uint32_t candidate[kCandidates][kMaxParts];  // indexes of samples
+  uint32_t equal[kCandidates][kMaxParts];
+  uint32_t cell2[kMaxCells];  // samples per cell by value
+  B wmin[kThreads / 32], wmax[kThreads / 32];
+  uint32_t wsum[kThreads / 32];
+  unsigned long long spread[2][kThreads / 32];
+  alignas(16) B sample[1];  // as many as the launch has room for
+};
+constexpr uint32_t kNone = 0xffffu, kWhole = 0xfffeu;  // no part; nor will there be one (the keys are equal)
+
+// Makes the map of src[0, len) for about k ranges: sm.tab and sm.part are its tables, `bins` its ranges (at most bin_room(k));
+// equal(bin, value) is called for each range that holds only keys equal to value. `salt` varies the sample. Every CTA that
+// calls it with the same arguments makes the same map.
+template <class T, class F>
+__device__ __forceinline__ void make_map(MapSmem<BOf<T>>& sm, const BOf<T>* src, uint32_t len, uint32_t k, uint32_t salt,
+                                         uint32_t over_sample, uint32_t max_sample, KeyMap<T>& map, uint32_t& bins, F&& equal) {
   using B = BOf<T>;
-  __shared__ B t[kMaxK];
-  __shared__ uint32_t cur[kMaxK];
-  __shared__ uint16_t lab[kMaxSlice];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t cells = cell_count(k);
+  uint32_t S = over_sample * k;
+  S = S < 1024u ? 1024u : S;
+  S = S > max_sample ? max_sample : S;
+  if (S > len) S = len;
+  const uint32_t step = len / S;
+  B mn = kmax<B>(), mx = B(0);
+#pragma unroll 8
+  for (uint32_t i = tid; i < S; i += kThreads) {
+    // one key at a pseudo-random place of each of S equal parts
+    uint32_t h = i * 2654435761u + salt * 40503u;
+    h ^= h >> 15;
+    h *= 0x85ebca6bu;
+    const uint32_t at = (uint32_t)(((unsigned long long)i * len) / S) + __umulhi(h, step);
+    const B x = KeyOps<T>::key(src[at]);
+    sm.sample[i] = x;
+    mn = x < mn ? x : mn;
+    mx = x > mx ? x : mx;
+  }
+  for (uint32_t i = tid; i < cells; i += kThreads) {
+    sm.tab[i] = 0u;
+    if (kFloating<T>) sm.cell2[i] = 0u;
+  }
+  mn = warp_min<B>(mn);
+  mx = warp_max<B>(mx);
+  if (lane == 0) {
+    sm.wmin[warp] = mn;
+    sm.wmax[warp] = mx;
+  }
+  __syncthreads();
+  mn = warp_min<B>(sm.wmin[lane & (kThreads / 32 - 1)]);
+  mx = warp_max<B>(sm.wmax[lane & (kThreads / 32 - 1)]);
+  // one cell more at each end, for the keys outside the sample's
+  map.lo = mn ? mn - 1u : mn;
+  const B hi = mx != kmax<B>() ? mx + 1u : mx;
+  map.span = hi - map.lo;
+  const int over = bits_of(map.span) - (31 - __clz(cells));
+  map.sh = over > 0 ? (uint32_t)over : 0u;
+  map.top = (uint32_t)(map.span >> map.sh);
+  map.used = map.top + 1u;
+  map.kind = 0u;
+  map.flo = map.scale = 0.f;
+  if (mn == mx) {  // one value (so far): the keys below, equal, above
+    bins = map.used;
+    map.kind = PARTS;  // for the mark
+    if (tid < map.used) sm.tab[tid] = tid | (map.lo + (B)tid == mn ? kEqual : 0u);
+    if (tid == 0) equal((uint32_t)(mn - map.lo), mn);
+    __syncthreads();
+    return;
+  }
+  for (uint32_t i = tid; i < S; i += kThreads) atomicAdd(&sm.tab[map.template cell<false>(sm.sample[i])], 1u);
+  if constexpr (kFloating<T>) {
+    KeyMap<T> other = map;
+    other.kind = BY_VALUE;
+    other.used = cells;
+    other.top = cells - 1u;
+    other.lo = mn;
+    other.span = mx - mn;
+    other.flo = as_float<T>(mn);
+    const float b = as_float<T>(mx), w = __fsub_rn(b, other.flo);
+    other.scale = __fdiv_rn((float)cells, w);
+    if (finite_span(other.flo, b, w) && other.scale < 3e38f) {  // the same in every thread
+      for (uint32_t i = tid; i < S; i += kThreads) atomicAdd(&sm.cell2[other.template cell<true>(sm.sample[i])], 1u);
+      __syncthreads();
+      unsigned long long sq[2] = {0ull, 0ull};
+      for (uint32_t i = tid; i < cells; i += kThreads) {
+        sq[0] += (unsigned long long)sm.tab[i] * sm.tab[i];
+        sq[1] += (unsigned long long)sm.cell2[i] * sm.cell2[i];
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) {
+        sq[0] += __shfl_xor_sync(0xffffffffu, sq[0], o);
+        sq[1] += __shfl_xor_sync(0xffffffffu, sq[1], o);
+      }
+      if (lane == 0) {
+        sm.spread[0][warp] = sq[0];
+        sm.spread[1][warp] = sq[1];
+      }
+      __syncthreads();
+      sq[0] = sq[1] = 0ull;
+      for (int i = 0; i < kThreads / 32; ++i) {
+        sq[0] += sm.spread[0][i];
+        sq[1] += sm.spread[1][i];
+      }
+      if (sq[1] < sq[0]) {
+        map = other;
+        for (uint32_t i = tid; i < cells; i += kThreads) sm.tab[i] = sm.cell2[i];
+      }
+    }
+  }
+  const bool by_value = kFloating<T> && map.kind;
+  __syncthreads();
+  // Cells with the sample of 1.5 ranges and more are divided, and their parts again, twice.
+  constexpr uint32_t R = kMaxCells / kThreads;
+  auto heavy = [&](uint32_t c) { return 2u * c * k >= 3u * S; };
+  uint32_t limit[4] = {0u, 0u, 0u, 0u};  // parts made by the end of each round
+  uint32_t first = 0u, end = cells, rounds = 0u;
+  for (uint32_t round = 0; round < 3u; ++round) {
+    const uint32_t per = (end - first + kThreads - 1u) / kThreads, e0 = first + tid * per;
+    uint32_t mine = 0u, total;
+    for (uint32_t i = 0; i < per; ++i) {
+      const uint32_t c = e0 + i < end ? sm.tab[e0 + i] : 0u;
+      if (heavy(c) && !(round && sm.node[e0 + i] == kWhole)) mine += (1u << 16) + min(4u * (c * k / S) + 4u, kPartSub);
+    }
+    uint32_t at = block_scan<kThreads>(mine, sm.wsum, total);
+    const uint32_t n0 = limit[round], n1 = min(n0 + (total >> 16), part_room(k));
+    if (n1 == n0) break;
+    ++rounds;
+    limit[round + 1u] = n1;
+    uint32_t last = min(end + (total & 0xffffu), cells + sub_room(k));
+    for (uint32_t i = 0; i < per; ++i) {
+      const uint32_t e = e0 + i;
+      if (e >= end) break;
+      const uint32_t c = sm.tab[e];
+      uint32_t node = kNone;
+      if (heavy(c) && !(round && sm.node[e] == kWhole)) {
+        const uint32_t sub = min(4u * (c * k / S) + 4u, kPartSub), p = n0 + (at >> 16), from = end + (at & 0xffffu);
+        at += (1u << 16) + sub;
+        if (p < n1) {
+          sm.entry[p] = e;
+          sm.part[p].sub = from;
+          sm.part[p].mult = from + sub <= last ? sub : 0u;  // 0: no room
+          sm.weight[p] = 0u;
+          sm.least[p] = ~0ull;
+          sm.greatest[p] = 0ull;
+#pragma unroll
+          for (int j = 0; j < kCandidates; ++j) {
+            sm.candidate[j][p] = ~0u;
+            sm.equal[j][p] = 0u;
+          }
+          if (from + sub <= last) node = p;
+        }
+      }
+      sm.node[e] = (uint16_t)node;
+    }
+    for (uint32_t i = end + tid; i < last; i += kThreads) {
+      sm.tab[i] = 0u;
+      sm.node[i] = (uint16_t)kNone;
+    }
+    __syncthreads();
+    // the part of this round that a sample is in, if it is less than kWhole
+    auto part_of = [&](B x) {
+      uint32_t e;
+      if (by_value) e = map.template cell<kFloating<T>>(x);
+      else e = map.template cell<false>(x);
+      uint32_t p = sm.node[e];
+      while (p < n0) p = sm.node[sm.part[p].of(x)];
+      return p;
+    };
+    for (uint32_t i = tid; i < S; i += kThreads) {
+      const uint32_t p = part_of(sm.sample[i]);
+      if (p >= kWhole) continue;
+      // the first samples of four parts of the sample: a frequent value most likely
+      atomicMin(&sm.candidate[i / kThreads % kCandidates][p], i);
+      atomicMin(&sm.least[p], (unsigned long long)sm.sample[i]);
+      atomicMax(&sm.greatest[p], (unsigned long long)sm.sample[i]);
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < S; i += kThreads) {
+      const B x = sm.sample[i];
+      const uint32_t p = part_of(x);
+      if (p >= kWhole) continue;
+#pragma unroll
+      for (int j = 0; j < kCandidates; ++j)
+        if (sm.candidate[j][p] != ~0u && x == sm.sample[sm.candidate[j][p]]) atomicAdd(&sm.equal[j][p], 1u);
+    }
+    __syncthreads();
+    for (uint32_t p = n0 + tid; p < n1; p += kThreads) {
+      Part<B> part = sm.part[p];
+      const uint32_t e = sm.entry[p], sub = part.mult;
+      if (!sub) continue;
+      uint32_t most = 0u;
+#pragma unroll
+      for (int j = 0; j < kCandidates; ++j)
+        if (sm.equal[j][p] > most) {
+          most = sm.equal[j][p];
+          part.lo = sm.sample[sm.candidate[j][p]];
+        }
+      if ((sm.tab[e] - most) * k <= S) {  // the others are a range at most
+        part.mult = 0u;
+        sm.weight[p] = 2u;
+        sm.node[part.sub + 1u] = (uint16_t)kWhole;
+      } else {
+        part.lo = (B)sm.least[p];
+        part.span = (B)sm.greatest[p] - part.lo;
+        const int bits = bits_of(part.span);
+        part.right = bits > 32 ? (uint32_t)bits - 32u : 0u;
+        part.left = bits < 32 ? 32u - (uint32_t)bits : 0u;
+        const unsigned long long top = (unsigned long long)((uint32_t)(part.span >> part.right) << part.left) + 1ull;
+        part.mult = (uint32_t)(((unsigned long long)sub << 32) / top);
+      }
+      sm.part[p] = part;
+      // the part that this one's cell is in: the last of the round before whose cells start at or before it
+      uint32_t o = kNone;
+      if (round)
+        for (uint32_t j = limit[round - 1u]; j < n0; ++j)
+          if (sm.node[sm.entry[j]] == j && sm.part[j].sub <= e) o = j;
+      sm.owner[p] = o;
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < S; i += kThreads) {
+      const B x = sm.sample[i];
+      const uint32_t p = part_of(x);
+      if (p < kWhole) atomicAdd(&sm.tab[sm.part[p].of(x)], 1u);
+    }
+    __syncthreads();
+    first = end;
+    end = last;
+  }
+  const uint32_t parts = limit[rounds];
+  if (!parts) {
+    const uint32_t per = cells > kThreads ? cells / kThreads : 1u, c0 = tid * per;
+    uint32_t c[R], sum = 0u, total;
+#pragma unroll
+    for (uint32_t r = 0; r < R; ++r) {
+      c[r] = r < per && c0 + r < cells ? sm.tab[c0 + r] : 0u;
+      sum += c[r];
+    }
+    uint32_t before = block_scan<kThreads>(sum, sm.wsum, total);
+#pragma unroll
+    for (uint32_t r = 0; r < R; ++r) {
+      if (r < per && c0 + r < cells) sm.tab[c0 + r] = before * k / S;
+      before += c[r];
+    }
+    bins = k + 1u;
+  } else {
+    // A range starts wherever k / S of the samples in front make a whole number; a single value's range is its own (one
+    // step before it and one behind it).
+    for (uint32_t p = tid; p < parts; p += kThreads)
+      if (sm.node[sm.entry[p]] == p && !sm.part[p].mult)
+        for (uint32_t o = sm.owner[p]; o != kNone; o = sm.owner[o]) atomicAdd(&sm.weight[o], 2u);
+    __syncthreads();
+    const uint32_t per = cells > kThreads ? cells / kThreads : 1u, c0 = tid * per;
+    auto sum_of = [&](uint32_t e) {
+      const uint32_t p = sm.node[e];
+      return sm.tab[e] + (p >= kWhole ? 0u : sm.weight[p] << 16);
+    };
+    auto settle = [&](uint32_t e, uint32_t before, uint32_t extra) {
+      const uint32_t p = sm.node[e];
+      if (p >= kWhole) {
+        sm.tab[e] = before * k / S + extra;
+      } else {
+        sm.tab[e] = 0x80000000u | p;
+        sm.before[p] = before;
+        sm.extra[p] = extra;
+      }
+    };
+    uint32_t sum = 0u, total;
+    for (uint32_t r = 0; r < per; ++r)
+      if (c0 + r < cells) sum += sum_of(c0 + r);
+    uint32_t at = block_scan<kThreads>(sum, sm.wsum, total);
+    for (uint32_t r = 0; r < per; ++r)
+      if (c0 + r < cells) {
+        const uint32_t c = sum_of(c0 + r);
+        settle(c0 + r, at & 0xffffu, at >> 16);
+        at += c;
+      }
+    for (uint32_t round = 0; round < rounds; ++round) {
+      __syncthreads();
+      for (uint32_t p = limit[round] + tid; p < limit[round + 1u]; p += kThreads) {
+        if (sm.tab[sm.entry[p]] != (0x80000000u | p)) continue;
+        const Part<B>& part = sm.part[p];
+        uint32_t in_front = sm.before[p] | (sm.extra[p] << 16);
+        const uint32_t sub = part.mult ? part.of(kmax<B>()) - part.sub + 1u : 3u;
+        for (uint32_t i = 0; i < sub; ++i) {
+          const uint32_t e = part.sub + i, c = sum_of(e);
+          settle(e, in_front & 0xffffu, in_front >> 16);
+          if (!part.mult && i == 1u) {
+            equal(sm.tab[e], part.lo);
+            sm.tab[e] |= kEqual;
+          }
+          in_front += c + (part.mult || i == 2u ? 0u : 1u << 16);
+        }
+      }
+    }
+    bins = k + 1u + (total >> 16);
+    map.kind |= PARTS | parts;
+    map.used = end;
+  }
+  __syncthreads();
+  if (!by_value && map.sh == 0u) {  // a range that is one cell of one value: nothing left to sort in it
+    bool any = false;
+    for (uint32_t i = tid; i <= map.top; i += kThreads) {
+      const uint32_t b = sm.tab[i];
+      auto apart = [&](uint32_t j) { return !(sm.tab[j] >> 31) && (sm.tab[j] & kBinMask) != b; };
+      if (b < kEqual && (i == 0u ? map.lo == B(0) : apart(i - 1u)) && (i == map.top ? hi == kmax<B>() : apart(i + 1u))) {
+        equal(b, map.lo + (B)i);
+        sm.tab[i] = b | kEqual;  // (the others compare what kBinMask leaves)
+        any = true;
+      }
+    }
+    if (__syncthreads_or(any)) map.kind |= PARTS;
+  }
+  __syncthreads();
+}
+
+template <class T>
+__global__ void __launch_bounds__(kThreads) split_map(const BOf<T>* src, Tables t, Level v, uint32_t plain_n, uint32_t levels,
+                                                      uint32_t max_sample, Queue* q) {
+  using B = BOf<T>;
+  extern __shared__ __align__(16) unsigned char split_dyn[];
+  MapSmem<B>& sm = *reinterpret_cast<MapSmem<B>*>(split_dyn);
+  const uint32_t tid = threadIdx.x;
   pdl_wait();
   pdl_trigger();
-  for (uint32_t i = threadIdx.x; i < k; i += kThreads) {
-    t[i] = tree[i];
-    cur[i] = 0u;
+  if (plain_n) {  // the first kernel of its sort, one CTA
+    clear(q, sizeof(Queue));
+    clear(t.ctl, sizeof(Ctl));
+    __threadfence();
+    __syncthreads();
   }
-  __syncthreads();
-  unsigned long long lo, hi;
-  slice_of(n, gridDim.x, lo, hi);  // hi - lo <= kMaxSlice (split_plan)
-  for (unsigned long long i0 = lo + threadIdx.x; i0 < hi; i0 += (unsigned long long)kBatch * kThreads) {
-    uint32_t b[kBatch];
-    B raw[kBatch];
-    buckets_of<T>(d, i0, hi, t, k, lg, b, raw);
+#ifdef GQS_PROFILE
+  if (tid == 0) atomicCAS(&q->lvl_start, 0ull, (unsigned long long)global_timer_ns());
+#endif
+  if (ld_relaxed(&q->error)) return;  // set before this grid started, if at all: the same for every thread
+  if (plain_n) {
+    if (tid == 0) add_segment(t, v, 0ull, plain_n, range_count<B>(plain_n, levels > 1u));
+    __threadfence();
+    __syncthreads();
+  }
+  const uint32_t nseg = (uint32_t)(__ldcg(&t.ctl->alloc[v.index]) >> 32);
+  for (uint32_t s = blockIdx.x; s < nseg; s += gridDim.x) {
+    SegRec* const rec = v.seg + s;
+    const uint32_t k = __ldcg(&rec->k), bin0 = __ldcg(&rec->bin0), cell0 = __ldcg(&rec->cell0);
+    for (uint32_t i = tid; i < bin_room(k); i += kThreads) {
+      v.bin[bin0 + i] = 0u;
+      v.eq[bin0 + i] = 0u;
+    }
+    KeyMap<T> map;
+    uint32_t bins;
+    make_map<T>(sm, src + __ldcg(&rec->start), __ldcg(&rec->len), k, s, SP_OVER, max_sample, map, bins, [&](uint32_t b, B x) {
+      v.eq[bin0 + b] = 1u;
+      v.value[bin0 + b] = x;
+    });
+    for (uint32_t i = tid; i < map.used; i += kThreads) v.cell[cell0 + i] = sm.tab[i];
+    Part<B>* const out = static_cast<Part<B>*>(v.part) + bin0 / 4u;
+    for (uint32_t i = tid; i < (map.kind & PART_COUNT); i += kThreads) out[i] = sm.part[i];
+    if (tid == 0) {
+      rec->lo = map.lo;
+      rec->span = map.span;
+      rec->sh = map.sh;
+      rec->used = map.used;
+      rec->top = map.top;
+      rec->kind = map.kind;
+      rec->flo = map.flo;
+      rec->scale = map.scale;
+      rec->bins = bins;
+    }
+    __syncthreads();
+  }
+}
+
+// ---- tiles of the segments of a level --------------------------------------------------------
+// The segment of tile `t`: the last one whose first tile is at most t.
+__device__ __forceinline__ uint32_t find_segment(const SegRec* seg, uint32_t nseg, uint32_t t) {
+  uint32_t lo = 0u, hi = nseg;
+  while (hi - lo > 1u) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (seg[mid].tile0 <= t) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+template <class T>
+__global__ void __launch_bounds__(kThreads, 3) split_count(const BOf<T>* src, Tables t, Level v, const Queue* q) {
+  using B = BOf<T>;
+  __shared__ uint32_t tab[kMaxCells + kMaxSub];
+  __shared__ uint32_t cnt[kBinSlots];
+  __shared__ Part<B> part[kMaxParts];
+  const uint32_t tid = threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
+  if (ld_relaxed(&q->error)) return;
+  const unsigned long long al = t.ctl->alloc[v.index];
+  const uint32_t tile_keys = t.tile_keys;
+  const uint32_t nseg = (uint32_t)(al >> 32), tiles = (uint32_t)al;
+  const uint32_t t0 = (uint32_t)((unsigned long long)tiles * blockIdx.x / gridDim.x);
+  const uint32_t t1 = (uint32_t)((unsigned long long)tiles * (blockIdx.x + 1u) / gridDim.x);
+  if (t0 >= t1) return;
+  uint32_t s = find_segment(v.seg, nseg, t0), tile = t0;
+  while (tile < t1) {
+    const SegRec r = v.seg[s];
+    const uint32_t seg_tiles = (r.len + tile_keys - 1u) / tile_keys;
+    const uint32_t end = r.tile0 + seg_tiles < t1 ? r.tile0 + seg_tiles : t1;
+    KeyMap<T> map;
+    map.load(r);
+    __syncthreads();
+    for (uint32_t i = tid; i < map.used; i += kThreads) tab[i] = v.cell[r.cell0 + i];
+    for (uint32_t i = tid; i < (map.kind & PART_COUNT); i += kThreads) part[i] = static_cast<const Part<B>*>(v.part)[r.bin0 / 4u + i];
+    for (uint32_t i = tid; i < r.bins; i += kThreads) cnt[i] = 0u;
+    __syncthreads();
+    // keys [k0, k1) of the segment
+    const uint32_t k0 = (tile - r.tile0) * tile_keys;
+    const uint32_t last = (end - r.tile0) * tile_keys, k1 = last < r.len ? last : r.len;
+    const B* const p = src + r.start;
+    by_kind<T>(map.kind, [&]<bool VALUE, bool PARTS_>() {
+      constexpr uint32_t U = 8;
+      uint32_t i = k0 + tid;
+      for (; i + (U - 1u) * kThreads < k1; i += U * kThreads) {
+        B x[U];
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      if (b[j] == kNone) continue;
-      lab[i0 + (unsigned long long)j * kThreads - lo] = (uint16_t)b[j];
-      atomicAdd(&cur[b[j]], 1u);
+        for (uint32_t u = 0; u < U; ++u) x[u] = p[i + u * kThreads];
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) atomicAdd(&cnt[map.template bin<VALUE, PARTS_>(KeyOps<T>::key(x[u]), tab, part) & kBinMask], 1u);
+      }
+      for (; i < k1; i += kThreads) atomicAdd(&cnt[map.template bin<VALUE, PARTS_>(KeyOps<T>::key(p[i]), tab, part) & kBinMask], 1u);
+    });
+    __syncthreads();
+    for (uint32_t b = tid; b < r.bins; b += kThreads)
+      if (cnt[b]) atomicAdd(&v.bin[r.bin0 + b], cnt[b]);
+    tile = end;
+    ++s;
+  }
+}
+
+// One CTA a segment: where every range starts; the ranges become records of the on-chip sort, or
+// segments of the next level.
+template <class T>
+__global__ void __launch_bounds__(kThreads) split_starts(Tables t, Level v, Level next, uint32_t levels, Queue* q) {
+  using B = BOf<T>;
+  __shared__ uint32_t wsum[kThreads / 32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u;
+  pdl_wait();
+  pdl_trigger();
+  if (ld_relaxed(&q->error)) return;
+  const uint32_t nseg = (uint32_t)(t.ctl->alloc[v.index] >> 32);
+  const bool more = v.index + 1u < levels;
+  const uint32_t side = v.index == 0u ? (uint32_t)IN_DN : 0u;
+  for (uint32_t s = blockIdx.x; s < nseg; s += gridDim.x) {
+    const SegRec r = v.seg[s];
+    if (tid == 0) {
+      atomicAdd(&q->part_keys, (unsigned long long)r.len);
+      atomicAdd(&q->part_jobs, 1u);
+      atomicMax(&q->max_depth, v.index);
+#ifdef GQS_PROFILE
+      level_note(q, v.index, 0, r.len);
+#endif
+    }
+    constexpr uint32_t R = (kBinSlots + kThreads - 1) / kThreads;
+    uint32_t c[R], sum = 0u, total;
+    bool still = false, moves = false;
+#pragma unroll
+    for (uint32_t i = 0; i < R; ++i) {
+      const uint32_t b = tid * R + i;
+      c[i] = b < r.bins ? __ldcg(&v.bin[r.bin0 + b]) : 0u;
+      sum += c[i];
+      if (!c[i]) continue;
+      if (!v.eq[r.bin0 + b]) moves = true;
+      else if (side && c[i] == r.len) still = true;
+    }
+    still = __syncthreads_or(still);
+    moves = __syncthreads_or(moves);
+    if (!moves && tid == 0) v.seg[s].bins = 0u;  // only equal keys: nothing to scatter
+    if (still) {                                 // of one value, and already in d
+      if (tid == 0) {
+        atomicAdd(&q->total, (unsigned long long)r.len);
+        atomicAdd(&q->done, (unsigned long long)r.len);
+      }
+      continue;
+    }
+    uint32_t at = block_scan<kThreads>(sum, wsum, total);
+#pragma unroll
+    for (uint32_t i = 0; i < R; ++i) {
+      const uint32_t b = tid * R + i;
+      const unsigned long long start = r.start + at;
+      const bool eq = c[i] && v.eq[r.bin0 + b];
+      if (b < r.bins) v.bin[r.bin0 + b] = at;
+      const bool split_again = !eq && more && c[i] > Sizes<B>::kLocal;
+      if (split_again && !add_segment(t, next, start, c[i], range_count<B>(c[i], false))) set_error(q, ST_INTERNAL, s);
+      const uint32_t recs = !c[i] || split_again ? 0u : eq ? (c[i] + kCopyChunk - 1u) / kCopyChunk : 1u;
+      uint32_t inc = recs;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+        if ((int)lane >= o) inc += u;
+      }
+      uint32_t first = 0u;
+      if (lane == 31 && inc) first = atomicAdd(&t.ctl->buckets, inc);
+      first = __shfl_sync(0xffffffffu, first, 31) + inc - recs;
+      for (uint32_t j = 0; j < recs; ++j) {
+        const uint32_t off = j * kCopyChunk;
+        t.bucket[first + j] = eq ? Bucket{start + off, c[i] - off < kCopyChunk ? c[i] - off : kCopyChunk, EQUAL, v.value[r.bin0 + b]}
+                                 : Bucket{start, c[i], side, 0ull};
+      }
+      at += c[i];
+    }
+    __syncthreads();
+  }
+}
+
+// ---- a tile's keys to their ranges --------------------------------------------------------------
+template <class B>
+struct TileSmem {
+  alignas(16) B keys[Sizes<B>::kTile];
+  uint32_t cnt[kBinSlots];
+  uint32_t gbase[kBinSlots];
+  uint32_t wsum[kThreads / 32];
+  uint16_t bin[Sizes<B>::kTile];
+};
+
+// One tile: `here` keys in registers (row j, thread tid: key j * kThreads + tid). Counts them by range with one shared atomic
+// each (its old value is the key's place in the tile's part of the range), reserves every range's share with reserve(range,
+// count), groups the keys by range in shared memory, calls between(), then puts each key with put(range, first, key, index):
+// the tile's part of the range is key indexes [.., ..) of the groups and starts at `first` - index of its first.
+// The reservation's round trip to L2 is hidden behind the grouping, the next tile's loads (between) behind the writes.
+template <class T, bool VALUE, bool PARTS_, bool COUNT_EQUAL, class Reserve, class Between, class Put>
+__device__ __forceinline__ void scatter_tile(TileSmem<BOf<T>>& sm, const KeyMap<T>& map, const uint32_t* tab, const Part<BOf<T>>* part,
+                                             uint32_t bins, const BOf<T> (&key)[Sizes<BOf<T>>::kTileRows], uint32_t here,
+                                             Reserve&& reserve, Between&& between, Put&& put) {
+  using B = BOf<T>;
+  constexpr int ROWS = Sizes<B>::kTileRows;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u;
+  uint32_t at[ROWS];  // (range << 16) | place in the tile's part of it; kLeft: left out
+  constexpr uint32_t kLeft = ~0u;
+  const bool full = !PARTS_ && here == (uint32_t)ROWS * kThreads;
+  uint32_t moved = here;
+  if (full) {
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) at[j] = map.template bin<VALUE, PARTS_>(key[j], tab, part);
+    // 32 adds to one counter run one by one: where rows seem to be of one range each, one add a row
+    const bool runs = __all_sync(0xffffffffu, at[0] == __shfl_sync(0xffffffffu, at[0], 0)) ||
+                      __all_sync(0xffffffffu, at[ROWS / 2] == __shfl_sync(0xffffffffu, at[ROWS / 2], 0));
+    if (!runs) {
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j) at[j] = (at[j] << 16) | atomicAdd(&sm.cnt[at[j]], 1u);
+    } else {
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j) {
+        const uint32_t b = at[j];
+        uint32_t rank = 0u;
+        if (__all_sync(0xffffffffu, b == __shfl_sync(0xffffffffu, b, 0))) {
+          if (lane == 0) rank = atomicAdd(&sm.cnt[b], 32u);
+          rank = __shfl_sync(0xffffffffu, rank, 0) + lane;
+        } else {
+          rank = atomicAdd(&sm.cnt[b], 1u);
+        }
+        at[j] = (b << 16) | rank;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+      at[j] = kLeft;
+      if ((uint32_t)j * kThreads + tid < here) {
+        const uint32_t b = map.template bin<VALUE, PARTS_>(key[j], tab, part);
+        if (!PARTS_ || b < kEqual) at[j] = (b << 16) | atomicAdd(&sm.cnt[b], 1u);
+        else if (COUNT_EQUAL) atomicAdd(&sm.cnt[b & kBinMask], 1u << 16);
+      }
     }
   }
   __syncthreads();
-  for (uint32_t b = threadIdx.x; b < k; b += kThreads)
-    if (cur[b]) cur[b] = atomicAdd(&cursor[b], cur[b]);
+  // range tid * per + i in thread tid; the first one's reservation is under way while the keys are grouped
+  const uint32_t per = (bins + kThreads - 1u) / kThreads, b0 = tid * per;
+  uint32_t base0 = 0u, ex0;
+  {
+    // in a counter: the keys to move, and above them those that are only counted
+    constexpr uint32_t kMoved = COUNT_EQUAL ? 0xffffu : ~0u;
+    auto all = [](uint32_t c) { return COUNT_EQUAL ? (c & 0xffffu) + (c >> 16) : c; };
+    uint32_t sum = 0u, total;
+    for (uint32_t i = 0; i < per; ++i)
+      if (b0 + i < bins) sum += sm.cnt[b0 + i] & kMoved;
+    const uint32_t c0 = b0 < bins ? sm.cnt[b0] : 0u;
+    if (c0) base0 = reserve(b0, all(c0));
+    ex0 = block_scan<kThreads>(sum, sm.wsum, total);
+    if (PARTS_) moved = total;
+    uint32_t ex = ex0;
+    for (uint32_t i = 0; i < per; ++i)
+      if (b0 + i < bins) {
+        const uint32_t c = sm.cnt[b0 + i];
+        sm.cnt[b0 + i] = ex;
+        if (i) sm.gbase[b0 + i] = c ? reserve(b0 + i, all(c)) - ex : 0u;
+        ex += c & kMoved;
+      }
+  }
   __syncthreads();
-  for (unsigned long long i0 = lo + threadIdx.x; i0 < hi; i0 += (unsigned long long)kBatch * kThreads) {
-    B raw[kBatch];
+  if (full) {
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      const unsigned long long i = i0 + (unsigned long long)j * kThreads;
-      raw[j] = i < hi ? d[i] : B(0);
+    for (int j = 0; j < ROWS; ++j) sm.keys[sm.cnt[at[j] >> 16] + (at[j] & 0xffffu)] = key[j];
+  } else {
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j)
+      if (at[j] != kLeft) {
+        const uint32_t i = sm.cnt[at[j] >> 16] + (at[j] & 0xffffu);
+        sm.keys[i] = key[j];
+        if (PARTS_) sm.bin[i] = (uint16_t)(at[j] >> 16);  // cheaper than to find it again
+      }
+  }
+  if (b0 < bins) sm.gbase[b0] = base0 - ex0;
+  between();
+  __syncthreads();
+  auto one = [&](uint32_t i) {
+    const B k = sm.keys[i];
+    const uint32_t b = PARTS_ ? sm.bin[i] : map.template bin<VALUE, PARTS_>(k, tab, part);
+    put(b, sm.gbase[b] + i, k);
+  };
+  if (full) {
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) one((uint32_t)j * kThreads + tid);
+  } else {
+#pragma unroll 1
+    for (uint32_t i = tid; i < moved; i += kThreads) one(i);
+  }
+}
+
+template <class B>
+struct ScatterSmem {
+  TileSmem<B> tile;
+  uint32_t tab[kMaxCells + kMaxSub];
+  Part<B> part[kMaxParts];
+};
+
+template <class T>
+__global__ void __launch_bounds__(kThreads, SP_MINB) split_scatter(const BOf<T>* src, BOf<T>* dst, Tables t, Level v, Queue* q) {
+  using B = BOf<T>;
+  constexpr int ROWS = Sizes<B>::kTileRows;
+  extern __shared__ __align__(16) unsigned char split_dyn[];
+  ScatterSmem<B>& sm = *reinterpret_cast<ScatterSmem<B>*>(split_dyn);
+  const uint32_t tid = threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
+  if (ld_relaxed(&q->error)) return;
+  const unsigned long long al = t.ctl->alloc[v.index];
+  const uint32_t tile_keys = t.tile_keys;
+  const uint32_t nseg = (uint32_t)(al >> 32), tiles = (uint32_t)al;
+  const uint32_t t0 = (uint32_t)((unsigned long long)tiles * blockIdx.x / gridDim.x);
+  const uint32_t t1 = (uint32_t)((unsigned long long)tiles * (blockIdx.x + 1u) / gridDim.x);
+  if (t0 >= t1) return;
+  uint32_t s = find_segment(v.seg, nseg, t0), seg_t0 = v.seg[s].tile0, seg_len = v.seg[s].len;
+  unsigned long long start = v.seg[s].start;
+  uint32_t bins = 0u, len;
+  uint32_t* cursor = nullptr;
+  B* out = nullptr;
+  KeyMap<T> map;
+  B key[ROWS];
+  auto load = [&](uint32_t tile) {
+    const uint32_t k0 = (tile - seg_t0) * tile_keys;
+    len = seg_len - k0 < tile_keys ? seg_len - k0 : tile_keys;
+    const B* const p = src + start + k0 + tid;
+    if (len == (uint32_t)ROWS * kThreads) {
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j) key[j] = KeyOps<T>::key(p[j * kThreads]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j)
+        if ((uint32_t)j * kThreads + tid < len) key[j] = KeyOps<T>::key(p[j * kThreads]);
     }
+  };
+  load(t0);
+  bool fresh = true;  // the tile is of another segment than the one before
+  auto advance = [&](uint32_t tile) {
+    fresh = false;
+    if (tile + 1u >= t1) return;
+    const uint32_t seg_end = seg_t0 + (seg_len + tile_keys - 1u) / tile_keys;
+    if (tile + 1u == seg_end) {
+      ++s;
+      seg_t0 = seg_end;
+      seg_len = v.seg[s].len;
+      start = v.seg[s].start;
+      fresh = true;
+    }
+    load(tile + 1u);
+  };
+  for (uint32_t tile = t0; tile < t1; ++tile) {
+    if (fresh) {
+      const SegRec* const r = v.seg + s;
+      map.load(*r);
+      bins = r->bins;
+      cursor = v.bin + r->bin0;
+      out = dst + start;
+      const uint32_t* const cell = v.cell + r->cell0;
+      __syncthreads();
+      for (uint32_t i = tid; i < map.used; i += kThreads) sm.tab[i] = cell[i];
+      for (uint32_t i = tid; i < (map.kind & PART_COUNT); i += kThreads) sm.part[i] = static_cast<const Part<B>*>(v.part)[r->bin0 / 4u + i];
+    }
+    if (!bins) {  // equal keys only, which need not move
+      advance(tile);
+      continue;
+    }
+    for (uint32_t i = tid; i < bins; i += kThreads) sm.tile.cnt[i] = 0u;
+    __syncthreads();
+    const uint32_t here = len;
+    B* const to = out;
+    uint32_t* const cur = cursor;
+    by_kind<T>(map.kind, [&]<bool VALUE, bool PARTS_>() {
+      scatter_tile<T, VALUE, PARTS_, false>(
+          sm.tile, map, sm.tab, sm.part, bins, key, here, [&](uint32_t b, uint32_t c) { return atomicAdd(cur + b, c); },
+          [&] { advance(tile); }, [&](uint32_t, uint32_t at, B k) { to[at] = KeyOps<T>::raw(k); });
+    });
+  }
+  if (tid == 0) atomicAdd(&q->chunks, (unsigned long long)(t1 - t0));
+}
+
+// ---- small plain sorts: map and scatter in one kernel, into ranges with room for kLocal keys each --------------
+template <class B>
+union SmallSmem {
+  char all[sizeof(MapSmem<B>) + Sizes<B>::kSmallSample * sizeof(B)];
+  MapSmem<B> map;
+  struct {
+    uint32_t tab[kMaxCells + kMaxSub];  // where the map leaves its tables
+    Part<B> part[kMaxParts];
+    TileSmem<B> tile;
+  } s;
+};
+
+template <class T>
+__global__ void __launch_bounds__(kThreads, SP_MINB) split_small(const BOf<T>* src, BOf<T>* area, uint32_t n, uint32_t k, Small* st, uint32_t tile_keys,
+                                                                 Queue* q) {
+  using B = BOf<T>;
+  constexpr int ROWS = Sizes<B>::kTileRows;
+  constexpr uint32_t LT = Sizes<B>::kLocal;
+  extern __shared__ __align__(16) unsigned char split_dyn[];
+  SmallSmem<B>& sm = *reinterpret_cast<SmallSmem<B>*>(split_dyn);
+  const uint32_t tid = threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
+  const uint32_t tiles = (n + tile_keys - 1u) / tile_keys;
+  KeyMap<T> map;
+  uint32_t bins;
+  if (blockIdx.x == 0) {
+    clear(q, sizeof(Queue));
+    clear(st->eq, bin_room(k) * 4);
+  }
+  make_map<T>(sm.map, src, n, k, 0u, kSmallOver, Sizes<B>::kSmallSample, map, bins, [&](uint32_t b, B x) {
+    if (blockIdx.x == 0) {
+      st->eq[b] = 1u;
+      st->value[b] = x;
+    }
+  });
+  if (blockIdx.x == 0 && tid == 0) {
+    st->bins = bins;
+    st->left = 0ull;
+    q->part_keys = n;
+    q->part_jobs = 1u;
+    q->chunks = tiles;
+#ifdef GQS_PROFILE
+    q->lvl_start = (unsigned long long)global_timer_ns();
+    level_note(q, 0, 0, n);
+#endif
+  }
+  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const uint32_t k0 = tile * tile_keys, here = n - k0 < tile_keys ? n - k0 : tile_keys;
+    B key[ROWS];
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      const unsigned long long i = i0 + (unsigned long long)j * kThreads;
-      if (i >= hi) continue;
-      const uint32_t pos = atomicAdd(&cur[lab[i - lo]], 1u);
-      dn[pos] = raw[j];  // pos < n: the bucket's reserved range holds exactly these keys
+    for (int j = 0; j < ROWS; ++j) {
+      const uint32_t i = (uint32_t)j * kThreads + tid;
+      if (i < here) key[j] = KeyOps<T>::key(src[k0 + i]);
+    }
+    for (uint32_t i = tid; i < bins; i += kThreads) sm.s.tile.cnt[i] = 0u;
+    __syncthreads();
+    by_kind<T>(map.kind, [&]<bool VALUE, bool PARTS_>() {
+      scatter_tile<T, VALUE, PARTS_, PARTS_>(
+          sm.s.tile, map, sm.s.tab, sm.s.part, bins, key, here,
+          [&](uint32_t b, uint32_t c) { return atomicAdd(&st->cursor[b], c); }, [] {},
+          [&](uint32_t b, uint32_t at, B x) {
+            // keys past the room are dropped: local_small sees that the range is too long and leaves the sort (its keys are
+            // still in d) to the persistent kernel
+            if (at < LT) area[(size_t)b * LT + at] = KeyOps<T>::raw(x);
+          });
+    });
+    __syncthreads();
+  }
+}
+
+// ---- the on-chip sort of a range ------------------------------------------------------------------
+// Sorting networks over registers (Batcher's odd-even merge).
+template <class K>
+__device__ __forceinline__ void order2(K& a, K& b) {
+  const K lo = a < b ? a : b, hi = a < b ? b : a;
+  a = lo;
+  b = hi;
+}
+template <class K>
+__device__ __forceinline__ void sort4(K* v) {
+  order2(v[0], v[1]); order2(v[2], v[3]);
+  order2(v[0], v[2]); order2(v[1], v[3]);
+  order2(v[1], v[2]);
+}
+template <class K>
+__device__ __forceinline__ void merge8(K* v) {  // v[0, 4) and v[4, 8) are sorted
+#pragma unroll
+  for (int i = 0; i < 4; ++i) order2(v[i], v[i + 4]);
+  order2(v[2], v[4]); order2(v[3], v[5]);
+  order2(v[1], v[2]); order2(v[3], v[4]); order2(v[5], v[6]);
+}
+template <class K>
+__device__ __forceinline__ void merge16(K* v) {  // v[0, 8) and v[8, 16) are sorted
+#pragma unroll
+  for (int i = 0; i < 8; ++i) order2(v[i], v[i + 8]);
+#pragma unroll
+  for (int i = 4; i < 8; ++i) order2(v[i], v[i + 4]);
+#pragma unroll
+  for (int i = 2; i < 12; i += 4) {
+    order2(v[i], v[i + 2]);
+    order2(v[i + 1], v[i + 3]);
+  }
+#pragma unroll
+  for (int i = 1; i < 15; i += 2) order2(v[i], v[i + 1]);
+}
+template <class K>
+__device__ __forceinline__ void sort16(K* v) {
+#pragma unroll
+  for (int h = 0; h < 16; h += 8) {
+    sort4(v + h);
+    sort4(v + h + 4);
+    merge8(v + h);
+  }
+  merge16(v);
+}
+
+template <class B>
+struct LocalSmem {
+  // Blocks of 16 keys, each followed by 16 bytes of padding, so that the lanes that read a block
+  // each with 16-byte loads meet different banks.
+  static constexpr uint32_t kPad = 16 / sizeof(B);
+  alignas(16) B keys[Sizes<B>::kLocal / 16 * (16 + kPad) + 64];
+  alignas(16) uint32_t cur[Sizes<B>::kLocal];
+  B wmin[Sizes<B>::kSortThreads / 32], wmax[Sizes<B>::kSortThreads / 32];
+  uint32_t wsum[Sizes<B>::kSortThreads / 32];
+  uint32_t most;
+  uint32_t todos;                                           // bins for a warp each
+  uint16_t todo[Sizes<B>::kLocal / (kShortBin + 1) + 2];
+  uint32_t bigs, big[Sizes<B>::kLocal / (kWarpBin + 1) + 1];  // bins for the CTA, later: (first key << 16) | keys
+  static __device__ __forceinline__ uint32_t slot(uint32_t i) { return i + (i >> 4) * kPad; }
+};
+
+// How a range's keys (less its least, mn) fall into bins: equal steps of the integer, or of the value.
+template <class T>
+struct BinMap {
+  using B = BOf<T>;
+  B mn;
+  uint32_t bins, sh, mult;  // (x >> sh) * mult / 2^32, or x itself (mult 0)
+  float flo, scale;
+  bool by_value;
+  __device__ __forceinline__ BinMap(B lo, B hi, uint32_t n, bool first) : mn(lo), bins(n), flo(0.f), scale(0.f), by_value(false) {
+    const B range = hi - lo;
+    const int over = bits_of(range) - 32;
+    sh = over > 0 ? (uint32_t)over : 0u;
+    const uint32_t top = (uint32_t)(range >> sh);
+    // rounded down far enough that no bin is past the last
+    mult = top < bins ? 0u : __float2uint_rz(__fmul_rn(__fdiv_rn((float)bins, __fadd_rn((float)top, 1.f)), 4294963200.f));
+    if constexpr (kFloating<T>) {
+      // keys on both sides of zero, or of many exponents: equal steps of the integer would leave most bins empty
+      constexpr int kExpShift = sizeof(B) == 8 ? 52 : 23;
+      const B zero = B(1) << (sizeof(B) * 8 - 1);
+      if (first && ((lo < zero && hi >= zero) || (range >> kExpShift) > 3u)) {
+        flo = as_float<T>(lo);
+        const float b = as_float<T>(hi), w = __fsub_rn(b, flo);
+        scale = __fdiv_rn((float)bins * 0.99999f, w);
+        by_value = finite_span(flo, b, w) && scale < 3e38f;
+      }
+    }
+  }
+  template <bool VALUE>
+  __device__ __forceinline__ uint32_t of(B x) const {
+    if constexpr (VALUE) {
+      const uint32_t u = __float2uint_rz(__fmul_rn(__fsub_rn(as_float<T>(x + mn), flo), scale));
+      return u < bins ? u : bins - 1u;
+    } else {
+      const uint32_t y = (uint32_t)(x >> sh);
+      return mult ? __umulhi(y, mult) : y;
+    }
+  }
+  __device__ __forceinline__ uint32_t any(B x) const {
+    if (kFloating<T> && by_value) return of<kFloating<T>>(x);
+    return of<false>(x);
+  }
+};
+
+// Sorts `len` keys (row j, thread tid: key j * NT + tid, as the map orders them) into dst[off, off + len). Calls between() once
+// the keys have left their registers. Every bin holds about one key, so after one counting pass each key is close to its place, and
+// networks over neighbouring blocks finish the order without knowing the bins.
+template <class T, class Between>
+__device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[Sizes<BOf<T>>::kLocalRows], uint32_t len, BOf<T>* dst,
+                                          uint32_t off, bool first, Between&& between) {
+  using B = BOf<T>;
+  using S = LocalSmem<B>;
+  constexpr int ROWS = Sizes<B>::kLocalRows;
+  constexpr uint32_t NT = Sizes<B>::kSortThreads, LT = Sizes<B>::kLocal;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  dst += off;
+  B mn = kmax<B>(), mx = B(0);
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j) {
+    if ((uint32_t)j * NT >= len) break;
+    if ((uint32_t)j * NT + tid < len) {
+      mn = key[j] < mn ? key[j] : mn;
+      mx = key[j] > mx ? key[j] : mx;
+    }
+  }
+  mn = warp_min<B>(mn);
+  mx = warp_max<B>(mx);
+  __syncthreads();  // the range before has left shared memory
+  if (lane == 0) {
+    sm.wmin[warp] = mn;
+    sm.wmax[warp] = mx;
+  }
+  // bins: a power of two, at least as many as keys
+  constexpr uint32_t kMinBins = 8u * NT < LT ? 8u * NT : LT;
+  const uint32_t bins = 1u << ceil_log2(len < kMinBins ? kMinBins : len);
+  for (uint32_t i = tid; i < bins / 4u; i += NT) reinterpret_cast<uint4*>(sm.cur)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (tid == 0) {
+    sm.most = 0u;
+    sm.todos = 0u;
+  }
+  __syncthreads();
+  mn = warp_min<B>(sm.wmin[lane & (NT / 32 - 1)]);
+  mx = warp_max<B>(sm.wmax[lane & (NT / 32 - 1)]);
+  const BinMap<T> map(mn, mx, bins, first);
+  auto count = [&]<bool VALUE>() {
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+      if ((uint32_t)j * NT >= len) break;
+      if ((uint32_t)j * NT + tid < len) {
+        key[j] -= mn;
+        atomicAdd(&sm.cur[map.template of<VALUE>(key[j])], 1u);
+      }
+    }
+  };
+  if (kFloating<T> && map.by_value) count.template operator()<kFloating<T>>();
+  else count.template operator()<false>();
+  __syncthreads();
+  {
+    // exclusive scan in place: a warp has bins / (NT / 32) consecutive counters, 256 at a time (8 a lane)
+    constexpr uint32_t CH = LT / (8u * NT);
+    uint4* const mine = reinterpret_cast<uint4*>(sm.cur) + warp * (bins / NT * 8u) + 2u * lane;
+    const uint32_t ch = bins / (8u * NT);
+    uint32_t before[CH], run = 0u, most = 0u;
+#pragma unroll
+    for (uint32_t i = 0; i < CH; ++i) {
+      if (i >= ch) break;
+      const uint4 c = mine[i * 64u], e = mine[i * 64u + 1u];
+      most = max(max(most, max(max(c.x, c.y), max(c.z, c.w))), max(max(e.x, e.y), max(e.z, e.w)));
+      const uint32_t sum = c.x + c.y + c.z + c.w + e.x + e.y + e.z + e.w;
+      uint32_t inc = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+        if ((int)lane >= o) inc += u;
+      }
+      before[i] = run + inc - sum;
+      run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) {
+      sm.wsum[warp] = run;
+      if (most > kShortBin) atomicMax(&sm.most, most);
+    }
+    __syncthreads();
+    const uint32_t up = __reduce_add_sync(0xffffffffu, lane < warp ? sm.wsum[lane] : 0u);
+#pragma unroll
+    for (uint32_t i = 0; i < CH; ++i) {
+      if (i >= ch) break;
+      const uint4 c = mine[i * 64u], e = mine[i * 64u + 1u];
+      uint4 v;
+      v.x = up + before[i];
+      v.y = v.x + c.x;
+      v.z = v.y + c.y;
+      v.w = v.z + c.z;
+      mine[i * 64u] = v;
+      v.x = v.w + c.w;
+      v.y = v.x + e.x;
+      v.z = v.y + e.y;
+      v.w = v.z + e.z;
+      mine[i * 64u + 1u] = v;
+    }
+  }
+  __syncthreads();
+  auto place = [&]<bool VALUE>() {
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+      if ((uint32_t)j * NT >= len) break;
+      if ((uint32_t)j * NT + tid < len) sm.keys[S::slot(atomicAdd(&sm.cur[map.template of<VALUE>(key[j])], 1u))] = key[j];
+    }
+  };
+  if (kFloating<T> && map.by_value) place.template operator()<kFloating<T>>();
+  else place.template operator()<false>();
+  const uint32_t blocks = (len + 15u) / 16u;
+  if (tid < blocks * 16u - len) sm.keys[S::slot(len + tid)] = kmax<B>();
+  const bool longs = sm.most > kShortBin;
+  between();
+  __syncthreads();
+  // cur[b] is now the end of bin b
+  if (longs) {
+    // Long bins: those of equal keys are in order as they are, the others are sorted by a warp each.
+    constexpr uint32_t kMixed = 0x80000000u;
+    auto first_of = [&](uint32_t b) { return b ? *(volatile uint32_t*)&sm.cur[b - 1u] & ~kMixed : 0u; };
+    auto end_of = [&](uint32_t b) { return *(volatile uint32_t*)&sm.cur[b] & ~kMixed; };
+    for (uint32_t i = tid; i < len; i += NT) {
+      const B k = sm.keys[S::slot(i)];
+      const uint32_t b = map.any(k), s = first_of(b);
+      if (end_of(b) - s > kShortBin && k != sm.keys[S::slot(s)] && !(atomicOr(&sm.cur[b], kMixed) >> 31)) {
+        const uint32_t n = end_of(b) - s;
+        if (n <= kWarpBin) sm.todo[atomicAdd(&sm.todos, 1u)] = (uint16_t)b;
+        else sm.big[atomicAdd(&sm.bigs, 1u)] = ((off + s) << 16) | n;
+      }
+    }
+    __syncthreads();
+    const uint32_t m = sm.todos;
+    for (uint32_t t = warp; t < m; t += NT / 32) {
+      const uint32_t b = sm.todo[t], s = first_of(b), n = end_of(b) - s;
+      auto sort_bin = [&]<int R>() {
+        B v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = r * 32u + lane < n ? sm.keys[S::slot(s + r * 32u + lane)] : kmax<B>();
+        warp_bitonic<R>(v);
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (lane * R + r < n) sm.keys[S::slot(s + lane * R + r)] = v[r];
+      };
+      if (n <= 32u) sort_bin.template operator()<1>();
+      else if (n <= 64u) sort_bin.template operator()<2>();
+      else if (n <= 128u) sort_bin.template operator()<4>();
+      else sort_bin.template operator()<8>();
+    }
+    __syncthreads();
+  }
+  // Every other key is within 8 places of its own: blocks of 16, then the halves that meet between them.
+  constexpr int V = 16 / (int)sizeof(B);
+  for (uint32_t b = tid; b < blocks; b += NT) {
+    B v[16];
+    uint4* const p = reinterpret_cast<uint4*>(&sm.keys[b * (16u + S::kPad)]);
+#pragma unroll
+    for (int i = 0; i < 16 / V; ++i) *reinterpret_cast<uint4*>(&v[i * V]) = p[i];
+    sort16(v);
+#pragma unroll
+    for (int i = 0; i < 16 / V; ++i) p[i] = *reinterpret_cast<const uint4*>(&v[i * V]);
+  }
+  __syncthreads();
+  for (uint32_t b = tid; b + 1u < blocks; b += NT) {
+    B v[16];
+    uint4* const p = reinterpret_cast<uint4*>(&sm.keys[b * (16u + S::kPad) + 8u]);
+    uint4* const r = reinterpret_cast<uint4*>(&sm.keys[(b + 1u) * (16u + S::kPad)]);
+#pragma unroll
+    for (int i = 0; i < 8 / V; ++i) {
+      *reinterpret_cast<uint4*>(&v[i * V]) = p[i];
+      *reinterpret_cast<uint4*>(&v[8 + i * V]) = r[i];
+    }
+    merge16(v);
+#pragma unroll
+    for (int i = 0; i < 8 / V; ++i) {
+      p[i] = *reinterpret_cast<const uint4*>(&v[i * V]);
+      r[i] = *reinterpret_cast<const uint4*>(&v[8 + i * V]);
+    }
+  }
+  __syncthreads();
+  for (uint32_t i = tid; i < len; i += NT) dst[i] = KeyOps<T>::raw(sm.keys[S::slot(i)] + mn);
+}
+
+template <class B>
+__device__ __forceinline__ void load_range(const B* p, uint32_t len, B (&raw)[Sizes<B>::kLocalRows]) {
+#pragma unroll
+  for (int j = 0; j < Sizes<B>::kLocalRows; ++j) {
+    if ((uint32_t)j * Sizes<B>::kSortThreads >= len) break;
+    if ((uint32_t)j * Sizes<B>::kSortThreads + threadIdx.x < len) raw[j] = p[j * Sizes<B>::kSortThreads + threadIdx.x];
+  }
+}
+
+// Sorts a range of `len` keys into dst (see sort_bins), with the longest bins that it leaves, each as a range of its own: its
+// two extremes fall into different bins then, of keys 2^11 times closer together, so there are at most six rounds.
+// Returns whether there were any (the keys that between() loaded are then lost).
+template <class T, class Between>
+__device__ __forceinline__ bool sort_range(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[Sizes<BOf<T>>::kLocalRows], uint32_t len, BOf<T>* dst,
+                                           Between&& between) {
+  using B = BOf<T>;
+  if (threadIdx.x == 0) sm.bigs = 0u;
+  sort_bins<T>(sm, key, len, dst, 0u, true, between);
+  if (sm.most <= kWarpBin) return false;
+  bool again = false;
+  while (true) {
+    __syncthreads();  // every thread has read what changes below, and sees the keys in dst
+    const uint32_t m = sm.bigs;
+    if (!m) return again;
+    again = true;
+    const uint32_t e = sm.big[m - 1u];
+    __syncthreads();
+    if (threadIdx.x == 0) sm.bigs = m - 1u;
+    load_range<B>(dst + (e >> 16), e & 0xffffu, key);
+#pragma unroll
+    for (int j = 0; j < Sizes<B>::kLocalRows; ++j) key[j] = KeyOps<T>::key(key[j]);
+    sort_bins<T>(sm, key, e & 0xffffu, dst, e >> 16, false, [] {});
+  }
+}
+
+template <class T>
+__global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<BOf<T>>::kSortCtas) local_sort(BOf<T>* d, BOf<T>* dn, unsigned long long n, Tables t, uint32_t plain_n, Queue* q) {
+  using B = BOf<T>;
+  constexpr int ROWS = Sizes<B>::kLocalRows;
+  constexpr uint32_t NT = Sizes<B>::kSortThreads, LT = Sizes<B>::kLocal;
+  extern __shared__ __align__(16) unsigned char split_dyn[];
+  LocalSmem<B>& sm = *reinterpret_cast<LocalSmem<B>*>(split_dyn);
+  const uint32_t tid = threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
+  if (plain_n) {  // the whole sort, by one CTA
+    clear(q, sizeof(Queue));
+    __threadfence();
+    __syncthreads();
+  } else if (ld_relaxed(&q->error)) {
+    return;
+  }
+#ifdef GQS_PROFILE
+  if (tid == 0) atomicCAS(&q->lvl_start, 0ull, (unsigned long long)global_timer_ns());
+#endif
+  const uint32_t nb = plain_n ? 1u : t.ctl->buckets;
+  unsigned long long sorted = 0ull, moved = 0ull;
+  uint32_t jobs = 0u;
+  B key[ROWS];
+  auto load = [&](const Bucket& k) {
+    if ((k.flags & EQUAL) || k.len > LT) return;
+    load_range<B>(((k.flags & IN_DN) ? dn : d) + k.start, k.len, key);
+  };
+  uint32_t at = blockIdx.x;
+  Bucket coming{};
+  if (at < nb) {
+    coming = plain_n ? Bucket{0ull, plain_n, 0u} : t.bucket[at];
+    load(coming);
+  }
+  for (; at < nb; at += gridDim.x) {
+    const Bucket bk = coming;
+    const bool more = at + gridDim.x < nb;
+    if (more) coming = t.bucket[at + gridDim.x];  // its keys are loaded once this range's have left the registers
+    if (!GQS_OK(bk.start + bk.len <= n, q, 0xD201ull)) break;
+    const B* const src = ((bk.flags & IN_DN) ? dn : d) + bk.start;
+    B* const dst = d + bk.start;
+    const uint32_t len = bk.len;
+    if ((bk.flags & EQUAL) || len > LT) {
+      bool same = (bk.flags & EQUAL) != 0u;
+      B x = KeyOps<T>::raw((B)bk.value);
+      // longer than the map's sample made likely: many equal keys, or keys too close together for it
+      if (!same && len <= 8u * kCopyChunk) {
+        x = src[0];
+        same = true;
+        for (uint32_t i0 = 0; i0 < len && same; i0 += 8u * NT) {
+          bool eq = true;
+#pragma unroll
+          for (uint32_t u = 0; u < 8u; ++u) {
+            const uint32_t i = i0 + u * NT + tid;
+            if (i < len) eq &= src[i] == x;
+          }
+          same = !__syncthreads_or(!eq);
+        }
+      }
+      if (same) {
+        for (uint32_t i = tid; i < len; i += NT) dst[i] = x;
+        moved += len;
+      } else if (tid == 0) {
+        const unsigned long long to = atomicAdd(&t.ctl->leftovers, 1ull);
+        t.left[2 * to] = bk.start;
+        t.left[2 * to + 1] = bk.start + len;
+        atomicAdd(&q->left, 1u);
+      }
+      if (more) load(coming);
+      continue;
+    }
+    sorted += len;
+    ++jobs;
+#ifdef GQS_PROFILE
+    if (tid == 0) level_note(q, 2u, 2, len);
+#endif
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+      if ((uint32_t)j * NT >= len) break;
+      key[j] = KeyOps<T>::key(key[j]);
+    }
+    const bool again = sort_range<T>(sm, key, len, dst, [&] {
+      if (more) load(coming);
+    });
+    if (again && more) load(coming);
+  }
+  if (tid == 0 && (sorted || moved)) {
+    atomicAdd(&q->total, sorted + moved);
+    atomicAdd(&q->done, sorted + moved);
+    if (jobs) {
+      atomicAdd(&q->local_keys, sorted);
+      atomicAdd(&q->local_jobs, jobs);
     }
   }
 }
 
-// Scratch layout: tree (kMaxK keys of 8 bytes), segment table (kMaxK + 1), totals, cursors.
-constexpr size_t kTreeBytes = kMaxK * 8;
-constexpr size_t kSegBytes = ((kMaxK + 1) * 8 + 255) / 256 * 256;
-constexpr size_t kCountBytes = kMaxK * 4;
+constexpr uint32_t kOwnRanges = 32;  // of one CTA of local_small
+struct Extent {
+  uint32_t bin, start, len;
+};
+template <class B>
+struct SmallSortSmem {
+  LocalSmem<B> local;
+  Extent own[kOwnRanges];
+  uint32_t wsum[Sizes<B>::kSortThreads / 32];
+  uint32_t fills;
+  Extent fill[Sizes<B>::kSmallMax / kCopyChunk + 1];  // long ranges of equal keys
+};
+
+// Every CTA of local_small calls this when it has read the cursors; the last one zeroes them.
+__device__ __forceinline__ void leave_small(Small* st, uint32_t bins) {
+  __threadfence();
+  if (__syncthreads_or(threadIdx.x == 0 && atomicAdd(&st->done, 1u) == gridDim.x - 1u)) {
+    for (uint32_t i = threadIdx.x; i < bins; i += blockDim.x) st->cursor[i] = 0u;
+    if (threadIdx.x == 0) st->done = 0u;
+  }
+}
+
+// The ranges of a small sort: their starts are the scan of their counts, which every CTA makes for itself.
+template <class T>
+__global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<BOf<T>>::kSortCtas) local_small(BOf<T>* d, const BOf<T>* area, uint32_t n, Small* st, Queue* q) {
+  using B = BOf<T>;
+  constexpr int ROWS = Sizes<B>::kLocalRows;
+  constexpr uint32_t NT = Sizes<B>::kSortThreads, LT = Sizes<B>::kLocal;
+  constexpr uint32_t R = (kBinSlots + NT - 1) / NT;
+  extern __shared__ __align__(16) unsigned char split_dyn[];
+  SmallSortSmem<B>& sm = *reinterpret_cast<SmallSortSmem<B>*>(split_dyn);
+  const uint32_t tid = threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
+  const uint32_t bins = st->bins;
+  uint32_t c[R], sum = 0u, total;
+  bool full = false;  // a range ran out of room
+  if (tid == 0) sm.fills = 0u;
+  __syncthreads();
+#pragma unroll
+  for (uint32_t i = 0; i < R; ++i) {
+    const uint32_t b = tid * R + i;
+    c[i] = b < bins ? st->cursor[b] : 0u;
+    if (c[i] > LT && !st->eq[b]) full = true;
+    sum += c[i];
+  }
+  if (__syncthreads_or(full)) {
+    if (blockIdx.x == 0 && tid == 0) {  // d is as it was: all of it is left to the persistent kernel
+      st->table[0] = 0ull;
+      st->table[1] = n;
+      st->left = 1ull;
+      q->left = 1u;
+    }
+    leave_small(st, bins);
+    return;
+  }
+  leave_small(st, bins);
+  uint32_t at = block_scan<NT>(sum, sm.wsum, total);
+#pragma unroll
+  for (uint32_t i = 0; i < R; ++i) {
+    const uint32_t b = tid * R + i;
+    if (b < bins && b % gridDim.x == blockIdx.x) sm.own[b / gridDim.x] = Extent{b, at, c[i]};
+    if (c[i] > kCopyChunk) sm.fill[atomicAdd(&sm.fills, 1u)] = Extent{b, at, c[i]};
+    at += c[i];
+  }
+  __syncthreads();
+  unsigned long long sorted = 0ull, moved = 0ull;
+  uint32_t jobs = 0u;
+  for (uint32_t o = 0; o * gridDim.x + blockIdx.x < bins; ++o) {
+    const uint32_t b = sm.own[o].bin, start = sm.own[o].start, len = sm.own[o].len;
+    if (!len || !GQS_OK(start + len <= n, q, 0xD202ull)) continue;
+    if (st->eq[b]) {
+      if (len <= kCopyChunk) {
+        const B x = KeyOps<T>::raw((B)st->value[b]);
+        for (uint32_t i = tid; i < len; i += NT) d[start + i] = x;
+      }
+      moved += len;  // longer ones below
+      continue;
+    }
+    sorted += len;
+    ++jobs;
+#ifdef GQS_PROFILE
+    if (tid == 0) level_note(q, 1u, 2, len);
+#endif
+    B key[ROWS];
+    load_range<B>(area + (size_t)b * LT, len, key);
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+      if ((uint32_t)j * NT >= len) break;
+      key[j] = KeyOps<T>::key(key[j]);
+    }
+    sort_range<T>(sm.local, key, len, d + start, [] {});
+  }
+  // long ranges of equal keys: every CTA writes a part of each
+  for (uint32_t f = 0; f < sm.fills; ++f) {
+    const uint32_t b = sm.fill[f].bin, start = sm.fill[f].start, len = sm.fill[f].len;
+    const B x = KeyOps<T>::raw((B)st->value[b]);
+    const uint32_t i0 = (uint32_t)((unsigned long long)len * blockIdx.x / gridDim.x);
+    const uint32_t i1 = (uint32_t)((unsigned long long)len * (blockIdx.x + 1u) / gridDim.x);
+    for (uint32_t i = i0 + tid; i < i1; i += NT) d[start + i] = x;
+  }
+  if (tid == 0 && (sorted || moved)) {
+    atomicAdd(&q->total, sorted + moved);
+    atomicAdd(&q->done, sorted + moved);
+    if (jobs) {
+      atomicAdd(&q->local_keys, sorted);
+      atomicAdd(&q->local_jobs, jobs);
+    }
+  }
+}
+
+// ---- host ----------------------------------------------------------------------------------------
+// Ranges of a small sort: few enough for one on each CTA of local_small where that leaves them short.
+template <class B>
+uint32_t small_count(size_t n, int sms) {
+  const size_t least = n / (Sizes<B>::kLocal / 10 * 3) + 1, most = n / 1024 + 1, want = (size_t)sms * Sizes<B>::kSortCtas;
+  const size_t k = want < least ? least : want > most ? most : want;
+  return k < 2 ? 2u : k > kMaxBins ? kMaxBins : (uint32_t)k;
+}
+
+template <class B>
+bool is_small(size_t n, bool plain) {
+  return plain && n > Sizes<B>::kLocal && n <= Sizes<B>::kSmallMax;
+}
+
+template <class B>
+struct Layout {
+  size_t segs[2], bins[2], cells[2], parts[2], buckets, left;
+  size_t ctl_at, seg_at[2], bin_at[2], eq_at[2], value_at[2], cell_at[2], part_at[2], bucket_at, left_at, small_at, area_at, bytes;
+  Layout(size_t n, size_t nseg, bool plain, int sms) {
+    const size_t L = Sizes<B>::kLocal, G = Sizes<B>::kTarget;
+    size_t at = 0;
+    auto put = [&at](size_t b) {
+      const size_t r = at;
+      at += (b + 255) / 256 * 256;
+      return r;
+    };
+    small_at = put(sizeof(Small));  // first, whatever n is: it has to stay as small sorts leave it
+    ctl_at = put(sizeof(Ctl));
+    left = n / L + 1;
+    left_at = put(left * 16);
+    if (is_small<B>(n, plain)) {
+      area_at = put((size_t)bin_room(small_count<B>(n, sms)) * L * sizeof(B));
+      bytes = at;
+      return;
+    }
+    segs[0] = plain ? 1 : n / L + 1;
+    segs[1] = n / L + 1;
+    for (int l = 0; l < 2; ++l) {
+      bins[l] = 5 * (n / G) / 2 + 9 * segs[l] + 8;
+      parts[l] = bins[l] / 4 + 1;
+      cells[l] = 16 * (n / G) + 312 * segs[l];
+      seg_at[l] = put(segs[l] * sizeof(SegRec));
+      bin_at[l] = put(bins[l] * 4);
+      eq_at[l] = put(bins[l] * 4);
+      value_at[l] = put(bins[l] * 8);
+      cell_at[l] = put(cells[l] * 4);
+      part_at[l] = put(parts[l] * sizeof(Part<B>));
+    }
+    buckets = bins[0] + bins[1] + n / kCopyChunk + (plain ? 0 : nseg) + 8;
+    bucket_at = put(buckets * sizeof(Bucket));
+    bytes = at;
+  }
+  Level level(void* scratch, int l) const {
+    char* p = static_cast<char*>(scratch);
+    return Level{reinterpret_cast<SegRec*>(p + seg_at[l]), reinterpret_cast<uint32_t*>(p + bin_at[l]),
+                 reinterpret_cast<unsigned long long*>(p + value_at[l]), reinterpret_cast<uint32_t*>(p + eq_at[l]), reinterpret_cast<uint32_t*>(p + cell_at[l]),
+                 p + part_at[l],
+                 (uint32_t)segs[l], (uint32_t)bins[l], (uint32_t)cells[l], (uint32_t)l};
+  }
+  Tables tables(void* scratch, uint32_t tile_keys) const {
+    char* p = static_cast<char*>(scratch);
+    return Tables{reinterpret_cast<Ctl*>(p + ctl_at), reinterpret_cast<Bucket*>(p + bucket_at),
+                  reinterpret_cast<unsigned long long*>(p + left_at), (uint32_t)buckets, tile_keys};
+  }
+};
+
+template <class K>
+cudaError_t allow_smem(K kernel, size_t bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
 
 template <class T>
-cudaError_t launch_t(const SplitPlan& p, const void* d, void* dn, size_t n, void* scratch, unsigned long long** segs,
-                     Queue* q, cudaStream_t s) {
+cudaError_t launch_t(const SplitArgs& a, SplitResult* out) {
   using B = BOf<T>;
-  char* base = static_cast<char*>(scratch);
-  B* tree = reinterpret_cast<B*>(base);
-  unsigned long long* sg = reinterpret_cast<unsigned long long*>(base + kTreeBytes);
-  uint32_t* total = reinterpret_cast<uint32_t*>(base + kTreeBytes + kSegBytes);
-  uint32_t* cursor = total + kMaxK;
-  const B* src = static_cast<const B*>(d);
-  constexpr size_t kPickSmem = 2 * kMaxSamples * sizeof(B);
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(split_pick<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPickSmem);
+  static const cudaError_t attr = [] {
+    cudaError_t e = allow_smem(split_scatter<T>, sizeof(ScatterSmem<B>));
+    if (e == cudaSuccess) e = allow_smem(split_map<T>, sizeof(MapSmem<B>) + Sizes<B>::kMaxSample * sizeof(B));
+    if (e == cudaSuccess) e = allow_smem(split_small<T>, sizeof(SmallSmem<B>));
+    if (e == cudaSuccess) e = allow_smem(local_sort<T>, sizeof(LocalSmem<B>));
+    if (e == cudaSuccess) e = allow_smem(local_small<T>, sizeof(SmallSortSmem<B>));
+    return e;
+  }();
   if (attr != cudaSuccess) return attr;
-  // Each kernel after the first is a programmatic dependent launch of the one before (and the
-  // seed and persistent kernels follow the same way), so that each launches while the one
-  // before it drains; split_pick also zeroes the bucket totals.
-  split_pick<T><<<1, kThreads, kPickSmem, s>>>(src, n, p.k, p.lg, p.samples, tree, total, q);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = launch_kernel(true, split_count<T>, dim3(p.ctas), dim3(kThreads), 0, s, src, (unsigned long long)n, p.k, p.lg,
-                      (const B*)tree, total);
-  if (e == cudaSuccess)
-    e = launch_kernel(true, split_starts, dim3(1), dim3(kMaxK), 0, s, (const uint32_t*)total, p.k,
-                      (unsigned long long)n, cursor, sg, q);
-  if (e == cudaSuccess)
-    e = launch_kernel(true, split_scatter<T>, dim3(p.ctas), dim3(kThreads), 0, s, src, static_cast<B*>(dn),
-                      (unsigned long long)n, p.k, p.lg, (const B*)tree, cursor);
-  *segs = sg;
+  const bool plain = a.offsets == nullptr;
+  const Layout<B> lay(a.n, a.nseg, plain, a.sms);
+  char* const base = static_cast<char*>(a.scratch);
+  B* d = static_cast<B*>(a.d);
+  B* dn = static_cast<B*>(a.dn);
+  cudaStream_t s = a.stream;
+  const uint32_t sms = (uint32_t)a.sms;
+  auto least = [](uint32_t x, size_t y) { return (size_t)x < y ? x : (uint32_t)y; };
+  cudaError_t e = cudaSuccess;
+  bool early = false;
+  auto go = [&](auto kernel, uint32_t grid, uint32_t block, size_t smem, auto... args) {
+    if (e == cudaSuccess) e = launch_kernel(early, kernel, dim3(grid), dim3(block), smem, s, args...);
+    early = true;
+  };
+  unsigned long long* const left = reinterpret_cast<unsigned long long*>(base + lay.left_at);
+  // tiles: large ones write longer runs; a small sort needs one for every SM
+  uint32_t tile_keys = Sizes<B>::kTile;
+  if (is_small<B>(a.n, plain)) {
+    while (tile_keys > 4u * kThreads && a.n / tile_keys < sms) tile_keys -= 2u * kThreads;
+    Small* st = reinterpret_cast<Small*>(base + lay.small_at);
+    B* area = reinterpret_cast<B*>(base + lay.area_at);
+    const uint32_t n = (uint32_t)a.n, tiles = (n + tile_keys - 1u) / tile_keys, k = small_count<B>(a.n, a.sms);
+    go(split_small<T>, least(sms * SP_MINB, tiles), kThreads, sizeof(SmallSmem<B>), (const B*)d, area, n, k, st, tile_keys, a.q);
+    const uint32_t ranges = bin_room(k), few = sms * Sizes<B>::kSortCtas, enough = (ranges + kOwnRanges - 1u) / kOwnRanges;
+    go(local_small<T>, few > ranges ? ranges : few > enough ? few : enough, Sizes<B>::kSortThreads, sizeof(SmallSortSmem<B>), d, (const B*)area, n, st, a.q);
+    out->table = reinterpret_cast<const unsigned long long*>(base + lay.small_at + offsetof(Small, table));
+    out->count = reinterpret_cast<const unsigned long long*>(base + lay.small_at + offsetof(Small, left));
+    out->most = 1u;
+    out->from_dn = 0u;
+    return e;
+  }
+  const uint32_t levels = a.n > (size_t)kMaxBins * Sizes<B>::kTarget || (plain && a.n > (1u << 21)) ? 2u : a.n > Sizes<B>::kLocal ? 1u : 0u;
+  while (tile_keys > 4u * kThreads && a.n / tile_keys < 2u * sms) tile_keys -= 2u * kThreads;
+  const Tables t = lay.tables(a.scratch, tile_keys);
+  const Level lv[2] = {lay.level(a.scratch, 0), lay.level(a.scratch, 1)};
+  if (!plain) {  // the first kernel of a plain sort clears them
+    e = cudaMemsetAsync(a.q, 0, sizeof(Queue), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(t.ctl, 0, sizeof(Ctl), s);
+    SortArgs<T> sa{};
+    sa.d = d;
+    sa.dn = dn;
+    sa.q = a.q;
+    sa.n = a.bound;
+    go(split_plan_segments<T>, (uint32_t)((a.nseg + 7) / 8), 256, 0, sa, t, lv[0], a.offsets, a.nseg_dev, (uint32_t)a.nseg, a.bound, a.pairs,
+       levels);
+  }
+  for (uint32_t l = 0; l < levels; ++l) {
+    const B* src = l ? dn : d;
+    B* dst = l ? d : dn;
+    const uint32_t gs = least(sms * 3u, lay.segs[l]);
+    const uint32_t tiles = (uint32_t)(a.n / tile_keys + lay.segs[l]);
+    const uint32_t sample = plain && !l ? Sizes<B>::kMaxSample : Sizes<B>::kMaxSample2;
+    go(split_map<T>, gs, kThreads, sizeof(MapSmem<B>) + sample * sizeof(B), src, t, lv[l], plain && !l ? (uint32_t)a.n : 0u, levels, sample, a.q);
+    go(split_count<T>, least(sms * 3u, tiles), kThreads, 0, src, t, lv[l], (const Queue*)a.q);
+    go(split_starts<T>, gs, kThreads, 0, t, lv[l], lv[1], levels, a.q);
+    go(split_scatter<T>, least(sms * SP_MINB, tiles), kThreads, sizeof(ScatterSmem<B>), src, dst, t, lv[l], a.q);
+  }
+  const bool one = plain && !levels;
+  go(local_sort<T>, one ? 1u : least(sms * Sizes<B>::kSortCtas, lay.buckets), Sizes<B>::kSortThreads, sizeof(LocalSmem<B>), d, dn, a.bound, t, one ? (uint32_t)a.n : 0u, a.q);
+  out->table = left;
+  out->count = &t.ctl->leftovers;
+  out->most = levels ? (uint32_t)lay.left : 0u;
+  out->from_dn = levels == 1u ? 1u : 0u;
   return e;
 }
 
 }  // namespace
 
-// Plain sorts of 2^15 .. 2^21 keys take the split (measured slower than the binary levels at
-// 2^22 on a GB300): k = the power of two that gives buckets of
-// about a third of a tile (so that nearly every bucket is one on-chip sort), at most kMaxK.
-bool split_plan(int dtype, size_t n, int tile, int sms, SplitPlan* plan) {
-  (void)dtype;
-  if (n < (1u << 15) || n > (1u << 21)) return false;
-  uint32_t k = 2, lg = 1;
-  while (k < kMaxK && (unsigned long long)k * (unsigned long long)tile < 3ull * n) {
-    k <<= 1;
-    ++lg;
-  }
-  plan->k = k;
-  plan->lg = lg;
-  plan->samples = k * kOversample < (uint32_t)kRun ? (uint32_t)kRun : k * kOversample;
-  if (plan->samples > kMaxSamples) plan->samples = kMaxSamples;
-  size_t ctas = n / 4096;  // about 4096 keys per CTA, at most two CTAs per SM ...
-  if (ctas > (size_t)(2 * sms)) ctas = (size_t)(2 * sms);
-  const size_t need = (n + kMaxSlice - 1) / kMaxSlice;  // ... and never more than kMaxSlice keys
-  if (ctas < need) ctas = need;
-  plan->ctas = (uint32_t)(ctas < 1 ? 1 : ctas);
-  return true;
+size_t split_scratch_bytes(int dtype, size_t n, size_t nseg, bool plain, int sms) {
+  return kDtypeBytes(dtype) == 4 ? Layout<uint32_t>(n, nseg, plain, sms).bytes : Layout<uint64_t>(n, nseg, plain, sms).bytes;
 }
 
-size_t split_scratch_bytes(const SplitPlan& plan) {
-  (void)plan;
-  return kTreeBytes + kSegBytes + 2 * kCountBytes;
-}
+size_t split_clear_bytes() { return sizeof(Small); }
 
-cudaError_t split_launch(int dtype, const SplitPlan& plan, const void* d, void* dn, size_t n, void* scratch,
-                         unsigned long long** segs, Queue* q, cudaStream_t s) {
+cudaError_t split_launch(int dtype, const SplitArgs& a, SplitResult* out) {
   switch (dtype) {
-    case DT_U32: return launch_t<uint32_t>(plan, d, dn, n, scratch, segs, q, s);
-    case DT_F32: return launch_t<float>(plan, d, dn, n, scratch, segs, q, s);
-    case DT_F64: return launch_t<double>(plan, d, dn, n, scratch, segs, q, s);
-    default: return launch_t<uint64_t>(plan, d, dn, n, scratch, segs, q, s);
+    case DT_U32: return launch_t<uint32_t>(a, out);
+    case DT_F32: return launch_t<float>(a, out);
+    case DT_F64: return launch_t<double>(a, out);
+    default: return launch_t<uint64_t>(a, out);
   }
 }
 
