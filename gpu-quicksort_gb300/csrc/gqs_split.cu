@@ -69,7 +69,6 @@ constexpr uint32_t kMaxCells = 4096;
 constexpr uint32_t kMaxParts = 256;             // cells divided further
 constexpr uint32_t kMaxSub = 2048;              // cells that those are divided into
 constexpr uint32_t kPartSub = 128;              // and at most so many for one
-constexpr uint32_t kShortBin = 9;               // longest bin that the networks of the on-chip sort put in order
 constexpr uint32_t kWarpBin = 256;              // longer ones of unequal keys are sorted by a warp each, beyond this by the CTA
 constexpr int kCandidates = 4;
 constexpr uint32_t kCopyChunk = 32768;          // keys of one record of a range of equal keys
@@ -83,6 +82,8 @@ struct Sizes {
   static constexpr int kTileRows = SP_KPT32 * 4 / (int)sizeof(B);
   static constexpr uint32_t kTile = kThreads * kTileRows;
   static constexpr int kLocalRows = (int)(kLocal / kSortThreads);
+  static constexpr int kBlock = sizeof(B) == 8 ? 8 : 16;     // keys of one network of the on-chip sort
+  static constexpr uint32_t kShortBin = kBlock / 2 + 1;      // longest bin that these put in order
   static constexpr uint32_t kTiny = sizeof(B) == 8 ? 128 : 256;
   // keys of a sample: at the first level of a plain sort (one CTA), at other levels, and in a small sort (two CTAs an SM)
   static constexpr uint32_t kMaxSample = sizeof(B) == 8 ? 16384 : 24576, kMaxSample2 = sizeof(B) == 8 ? 8192 : 12288;
@@ -1198,32 +1199,63 @@ __device__ __forceinline__ void merge16(K* v) {  // v[0, 8) and v[8, 16) are sor
 #pragma unroll
   for (int i = 1; i < 15; i += 2) order2(v[i], v[i + 1]);
 }
-template <class K>
-__device__ __forceinline__ void sort16(K* v) {
+template <int W, class K>
+__device__ __forceinline__ void merge_block(K* v) {
+  static_assert(W == 8 || W == 16, "networks of 8 and 16 keys");
+  if constexpr (W == 8) merge8(v);
+  else merge16(v);
+}
+template <int W, class K>
+__device__ __forceinline__ void sort_block(K* v) {
 #pragma unroll
-  for (int h = 0; h < 16; h += 8) {
+  for (int h = 0; h < W; h += 8) {
     sort4(v + h);
     sort4(v + h + 4);
     merge8(v + h);
   }
-  merge16(v);
+  if constexpr (W == 16) merge16(v);
 }
 
 template <class B>
 struct LocalSmem {
-  // Blocks of 16 keys, each followed by 16 bytes of padding, so that the lanes that read a block
-  // each with 16-byte loads meet different banks.
-  static constexpr uint32_t kPad = 16 / sizeof(B);
-  alignas(16) B keys[Sizes<B>::kLocal / 16 * (16 + kPad) + 64];
-  alignas(16) uint32_t cur[Sizes<B>::kLocal];
+  // Blocks of kBlock keys. The 16-byte pieces of each are permuted by its number, so that eight lanes that read the same piece of
+  // neighbouring blocks meet different banks.
+  alignas(128) B keys[Sizes<B>::kLocal];
+  alignas(16) uint32_t cur[Sizes<B>::kLocal / 2];  // the bins' counters, two in each word
   B wmin[Sizes<B>::kSortThreads / 32], wmax[Sizes<B>::kSortThreads / 32];
   uint32_t wsum[Sizes<B>::kSortThreads / 32];
   uint32_t most;
   uint32_t todos;                                           // bins for a warp each
-  uint16_t todo[Sizes<B>::kLocal / (kShortBin + 1) + 2];
+  uint16_t todo[Sizes<B>::kLocal / (Sizes<B>::kShortBin + 1) + 2];
   uint32_t bigs, big[Sizes<B>::kLocal / (kWarpBin + 1) + 1];  // bins for the CTA, later: (first key << 16) | keys
-  static __device__ __forceinline__ uint32_t slot(uint32_t i) { return i + (i >> 4) * kPad; }
+  static constexpr uint32_t V = 16 / sizeof(B), kPieces = Sizes<B>::kBlock / V;  // keys of a piece, pieces of a block
+  static __device__ __forceinline__ uint32_t slot(uint32_t i) { return i ^ ((i / V >> 3 & (kPieces - 1u)) * V); }
+  __device__ __forceinline__ uint4* piece(uint32_t b, uint32_t i) {
+    return reinterpret_cast<uint4*>(keys) + (b * kPieces + i ^ (b * kPieces >> 3 & (kPieces - 1u)));
+  }
 };
+
+// f(j) for every row j, of NT keys each, in which this thread has one of `len` keys: four full rows at a time need no test for each.
+// (Recursion, not a loop: around a loop that ends early the compiler kept the keys in local memory.)
+template <int ROWS, uint32_t NT, int J = 0, class F>
+__device__ __forceinline__ void for_rows(uint32_t len, F&& f) {
+  static_assert(ROWS % 4 == 0, "whole groups");
+  if constexpr (J < ROWS) {
+    if ((uint32_t)(J + 4) * NT <= len) {
+      f(J);
+      f(J + 1);
+      f(J + 2);
+      f(J + 3);
+      for_rows<ROWS, NT, J + 4>(len, f);
+    } else {
+      const uint32_t i = (uint32_t)J * NT + threadIdx.x;
+      if (i < len) f(J);
+      if (i + NT < len) f(J + 1);
+      if (i + 2u * NT < len) f(J + 2);
+      if (i + 3u * NT < len) f(J + 3);
+    }
+  }
+}
 
 // How a range's keys (less its least, mn) fall into bins: equal steps of the integer, or of the value.
 template <class T>
@@ -1277,18 +1309,15 @@ __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[S
   using B = BOf<T>;
   using S = LocalSmem<B>;
   constexpr int ROWS = Sizes<B>::kLocalRows;
-  constexpr uint32_t NT = Sizes<B>::kSortThreads, LT = Sizes<B>::kLocal;
+  constexpr uint32_t NT = Sizes<B>::kSortThreads, LT = Sizes<B>::kLocal, kShortBin = Sizes<B>::kShortBin;
+  constexpr int W = Sizes<B>::kBlock;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   dst += off;
   B mn = kmax<B>(), mx = B(0);
-#pragma unroll
-  for (int j = 0; j < ROWS; ++j) {
-    if ((uint32_t)j * NT >= len) break;
-    if ((uint32_t)j * NT + tid < len) {
-      mn = key[j] < mn ? key[j] : mn;
-      mx = key[j] > mx ? key[j] : mx;
-    }
-  }
+  for_rows<ROWS, NT>(len, [&](int j) {
+    mn = key[j] < mn ? key[j] : mn;
+    mx = key[j] > mx ? key[j] : mx;
+  });
   mn = warp_min<B>(mn);
   mx = warp_max<B>(mx);
   __syncthreads();  // the range before has left shared memory
@@ -1298,8 +1327,9 @@ __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[S
   }
   // bins: a power of two, at least as many as keys
   constexpr uint32_t kMinBins = 8u * NT < LT ? 8u * NT : LT;
-  const uint32_t bins = 1u << ceil_log2(len < kMinBins ? kMinBins : len);
-  for (uint32_t i = tid; i < bins / 4u; i += NT) reinterpret_cast<uint4*>(sm.cur)[i] = make_uint4(0u, 0u, 0u, 0u);
+  const uint32_t some = 16u / W * len;
+  const uint32_t bins = 1u << ceil_log2(some < kMinBins ? kMinBins : some < LT ? some : LT);
+  for (uint32_t i = tid; i < bins / 8u; i += NT) reinterpret_cast<uint4*>(sm.cur)[i] = make_uint4(0u, 0u, 0u, 0u);
   if (tid == 0) {
     sm.most = 0u;
     sm.todos = 0u;
@@ -1309,30 +1339,29 @@ __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[S
   mx = warp_max<B>(sm.wmax[lane & (NT / 32 - 1)]);
   const BinMap<T> map(mn, mx, bins, first);
   auto count = [&]<bool VALUE>() {
-#pragma unroll
-    for (int j = 0; j < ROWS; ++j) {
-      if ((uint32_t)j * NT >= len) break;
-      if ((uint32_t)j * NT + tid < len) {
-        key[j] -= mn;
-        atomicAdd(&sm.cur[map.template of<VALUE>(key[j])], 1u);
-      }
-    }
+    for_rows<ROWS, NT>(len, [&](int j) {
+      key[j] -= mn;
+      const uint32_t b = map.template of<VALUE>(key[j]);
+      atomicAdd(&sm.cur[b >> 1], b & 1u ? 0x10000u : 1u);
+    });
   };
   if (kFloating<T> && map.by_value) count.template operator()<kFloating<T>>();
   else count.template operator()<false>();
   __syncthreads();
   {
-    // exclusive scan in place: a warp has bins / (NT / 32) consecutive counters, 256 at a time (8 a lane)
+    // exclusive scan in place: a warp has bins / (NT / 32) consecutive counters, 256 at a time (8 a lane, in one 16-byte word)
     constexpr uint32_t CH = LT / (8u * NT);
-    uint4* const mine = reinterpret_cast<uint4*>(sm.cur) + warp * (bins / NT * 8u) + 2u * lane;
+    uint4* const mine = reinterpret_cast<uint4*>(sm.cur) + warp * (bins / NT * 4u) + lane;
     const uint32_t ch = bins / (8u * NT);
     uint32_t before[CH], run = 0u, most = 0u;
+    // halves of x: c0 and c1; of pair(x): c0 and c0 + c1
+    auto pair = [](uint32_t x) { return x * 0x10001u; };
 #pragma unroll
     for (uint32_t i = 0; i < CH; ++i) {
       if (i >= ch) break;
-      const uint4 c = mine[i * 64u], e = mine[i * 64u + 1u];
-      most = max(max(most, max(max(c.x, c.y), max(c.z, c.w))), max(max(e.x, e.y), max(e.z, e.w)));
-      const uint32_t sum = c.x + c.y + c.z + c.w + e.x + e.y + e.z + e.w;
+      const uint4 w = mine[i * 32u];
+      most = __vmaxu2(most, __vmaxu2(__vmaxu2(w.x, w.y), __vmaxu2(w.z, w.w)));
+      const uint32_t sum = pair(w.x + w.y + w.z + w.w) >> 16;  // (at most kLocal: no half carries into the other)
       uint32_t inc = sum;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -1342,7 +1371,7 @@ __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[S
       before[i] = run + inc - sum;
       run += __shfl_sync(0xffffffffu, inc, 31);
     }
-    most = __reduce_max_sync(0xffffffffu, most);
+    most = __reduce_max_sync(0xffffffffu, max(most >> 16, most & 0xffffu));
     if (lane == 0) {
       sm.wsum[warp] = run;
       if (most > kShortBin) atomicMax(&sm.most, most);
@@ -1352,45 +1381,52 @@ __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[S
 #pragma unroll
     for (uint32_t i = 0; i < CH; ++i) {
       if (i >= ch) break;
-      const uint4 c = mine[i * 64u], e = mine[i * 64u + 1u];
+      uint32_t e = pair(up + before[i]);  // in both halves
+      auto next = [&](uint32_t x) {
+        const uint32_t v = e + (x << 16);
+        e += pair(pair(x) >> 16);
+        return v;
+      };
+      const uint4 w = mine[i * 32u];
       uint4 v;
-      v.x = up + before[i];
-      v.y = v.x + c.x;
-      v.z = v.y + c.y;
-      v.w = v.z + c.z;
-      mine[i * 64u] = v;
-      v.x = v.w + c.w;
-      v.y = v.x + e.x;
-      v.z = v.y + e.y;
-      v.w = v.z + e.z;
-      mine[i * 64u + 1u] = v;
+      v.x = next(w.x);
+      v.y = next(w.y);
+      v.z = next(w.z);
+      v.w = next(w.w);
+      mine[i * 32u] = v;
     }
   }
   __syncthreads();
   auto place = [&]<bool VALUE>() {
-#pragma unroll
-    for (int j = 0; j < ROWS; ++j) {
-      if ((uint32_t)j * NT >= len) break;
-      if ((uint32_t)j * NT + tid < len) sm.keys[S::slot(atomicAdd(&sm.cur[map.template of<VALUE>(key[j])], 1u))] = key[j];
-    }
+    for_rows<ROWS, NT>(len, [&](int j) {
+      const uint32_t b = map.template of<VALUE>(key[j]);
+      const uint32_t old = atomicAdd(&sm.cur[b >> 1], b & 1u ? 0x10000u : 1u);
+      sm.keys[S::slot(b & 1u ? old >> 16 : old & 0xffffu)] = key[j];
+    });
   };
   if (kFloating<T> && map.by_value) place.template operator()<kFloating<T>>();
   else place.template operator()<false>();
-  const uint32_t blocks = (len + 15u) / 16u;
-  if (tid < blocks * 16u - len) sm.keys[S::slot(len + tid)] = kmax<B>();
+  const uint32_t blocks = (len + W - 1u) / W;
+  if (tid < blocks * W - len) sm.keys[S::slot(len + tid)] = kmax<B>();
   const bool longs = sm.most > kShortBin;
   between();
   __syncthreads();
   // cur[b] is now the end of bin b
   if (longs) {
     // Long bins: those of equal keys are in order as they are, the others are sorted by a warp each.
-    constexpr uint32_t kMixed = 0x80000000u;
-    auto first_of = [&](uint32_t b) { return b ? *(volatile uint32_t*)&sm.cur[b - 1u] & ~kMixed : 0u; };
-    auto end_of = [&](uint32_t b) { return *(volatile uint32_t*)&sm.cur[b] & ~kMixed; };
+    constexpr uint32_t kMixed = 0x8000u;
+    static_assert(LT < kMixed, "a counter's bits below the mark");
+    volatile uint16_t* const ends = reinterpret_cast<volatile uint16_t*>(sm.cur);
+    auto end_of = [&](uint32_t b) { return ends[b] & (kMixed - 1u); };
+    auto first_of = [&](uint32_t b) { return b ? end_of(b - 1u) : 0u; };
+    auto mark = [&](uint32_t b) {  // whether it was marked before
+      const uint32_t m = kMixed << (16u * (b & 1u));
+      return (atomicOr(&sm.cur[b >> 1], m) & m) != 0u;
+    };
     for (uint32_t i = tid; i < len; i += NT) {
       const B k = sm.keys[S::slot(i)];
       const uint32_t b = map.any(k), s = first_of(b);
-      if (end_of(b) - s > kShortBin && k != sm.keys[S::slot(s)] && !(atomicOr(&sm.cur[b], kMixed) >> 31)) {
+      if (end_of(b) - s > kShortBin && k != sm.keys[S::slot(s)] && !mark(b)) {
         const uint32_t n = end_of(b) - s;
         if (n <= kWarpBin) sm.todo[atomicAdd(&sm.todos, 1u)] = (uint16_t)b;
         else sm.big[atomicAdd(&sm.bigs, 1u)] = ((off + s) << 16) | n;
@@ -1417,44 +1453,55 @@ __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[S
     }
     __syncthreads();
   }
-  // Every other key is within 8 places of its own: blocks of 16, then the halves that meet between them.
-  constexpr int V = 16 / (int)sizeof(B);
+  // Every other key is within W / 2 places of its own: blocks of W, then the halves that meet between them.
+  constexpr int V = S::V, P = W / V;
   for (uint32_t b = tid; b < blocks; b += NT) {
-    B v[16];
-    uint4* const p = reinterpret_cast<uint4*>(&sm.keys[b * (16u + S::kPad)]);
+    B v[W];
 #pragma unroll
-    for (int i = 0; i < 16 / V; ++i) *reinterpret_cast<uint4*>(&v[i * V]) = p[i];
-    sort16(v);
+    for (int i = 0; i < P; ++i) *reinterpret_cast<uint4*>(&v[i * V]) = *sm.piece(b, i);
+    sort_block<W>(v);
 #pragma unroll
-    for (int i = 0; i < 16 / V; ++i) p[i] = *reinterpret_cast<const uint4*>(&v[i * V]);
+    for (int i = 0; i < P; ++i) *sm.piece(b, i) = *reinterpret_cast<const uint4*>(&v[i * V]);
   }
   __syncthreads();
   for (uint32_t b = tid; b + 1u < blocks; b += NT) {
-    B v[16];
-    uint4* const p = reinterpret_cast<uint4*>(&sm.keys[b * (16u + S::kPad) + 8u]);
-    uint4* const r = reinterpret_cast<uint4*>(&sm.keys[(b + 1u) * (16u + S::kPad)]);
+    B v[W];
 #pragma unroll
-    for (int i = 0; i < 8 / V; ++i) {
-      *reinterpret_cast<uint4*>(&v[i * V]) = p[i];
-      *reinterpret_cast<uint4*>(&v[8 + i * V]) = r[i];
+    for (int i = 0; i < P / 2; ++i) {
+      *reinterpret_cast<uint4*>(&v[i * V]) = *sm.piece(b, P / 2 + i);
+      *reinterpret_cast<uint4*>(&v[W / 2 + i * V]) = *sm.piece(b + 1u, i);
     }
-    merge16(v);
+    merge_block<W>(v);
 #pragma unroll
-    for (int i = 0; i < 8 / V; ++i) {
-      p[i] = *reinterpret_cast<const uint4*>(&v[i * V]);
-      r[i] = *reinterpret_cast<const uint4*>(&v[8 + i * V]);
+    for (int i = 0; i < P / 2; ++i) {
+      *sm.piece(b, P / 2 + i) = *reinterpret_cast<const uint4*>(&v[i * V]);
+      *sm.piece(b + 1u, i) = *reinterpret_cast<const uint4*>(&v[W / 2 + i * V]);
     }
   }
   __syncthreads();
-  for (uint32_t i = tid; i < len; i += NT) dst[i] = KeyOps<T>::raw(sm.keys[S::slot(i)] + mn);
+  const B* const mine = &sm.keys[S::slot(tid)];
+  static_assert(NT % 128u == 0u, "slot(i + NT) is slot(i) + NT");
+  B* const to = dst + tid;
+  for_rows<ROWS, NT>(len, [&](int j) { to[j * NT] = KeyOps<T>::raw(mine[j * NT] + mn); });
+}
+
+// v = *p where `use`: as inline code, so that the loads stay one behind the other with nothing between them.
+__device__ __forceinline__ void load_if(uint32_t& v, const uint32_t* p, bool use) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q ld.global.u32 %0, [%1];\n}" : "+r"(v) : "l"(p), "r"((uint32_t)use) : "memory");
+}
+__device__ __forceinline__ void load_if(uint64_t& v, const uint64_t* p, bool use) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q ld.global.u64 %0, [%1];\n}" : "+l"(v) : "l"(p), "r"((uint32_t)use) : "memory");
 }
 
 template <class B>
 __device__ __forceinline__ void load_range(const B* p, uint32_t len, B (&raw)[Sizes<B>::kLocalRows]) {
+  const B* const mine = p + threadIdx.x;
 #pragma unroll
-  for (int j = 0; j < Sizes<B>::kLocalRows; ++j) {
+  for (int j = 0; j < Sizes<B>::kLocalRows; j += 4) {
     if ((uint32_t)j * Sizes<B>::kSortThreads >= len) break;
-    if ((uint32_t)j * Sizes<B>::kSortThreads + threadIdx.x < len) raw[j] = p[j * Sizes<B>::kSortThreads + threadIdx.x];
+#pragma unroll
+    for (int u = j; u < j + 4; ++u)
+      load_if(raw[u], mine + u * Sizes<B>::kSortThreads, (uint32_t)u * Sizes<B>::kSortThreads + threadIdx.x < len);
   }
 }
 
@@ -1478,10 +1525,24 @@ __device__ __forceinline__ bool sort_range(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[
     __syncthreads();
     if (threadIdx.x == 0) sm.bigs = m - 1u;
     load_range<B>(dst + (e >> 16), e & 0xffffu, key);
-#pragma unroll
-    for (int j = 0; j < Sizes<B>::kLocalRows; ++j) key[j] = KeyOps<T>::key(key[j]);
+    for_rows<Sizes<B>::kLocalRows, Sizes<B>::kSortThreads>(e & 0xffffu, [&](int j) { key[j] = KeyOps<T>::key(key[j]); });
     sort_bins<T>(sm, key, e & 0xffffu, dst, e >> 16, false, [] {});
   }
+}
+
+// p[0, len) = x, by nt threads
+template <class B>
+__device__ __forceinline__ void fill_range(B* p, uint32_t len, B x, uint32_t tid, uint32_t nt) {
+  constexpr uint32_t V = 16 / sizeof(B);
+  const uint32_t over = (uint32_t)(-(reinterpret_cast<uintptr_t>(p) / sizeof(B)) & (V - 1u)), head = over < len ? over : len;
+  const uint32_t vecs = (len - head) / V;
+  if (tid < head) p[tid] = x;
+  uint4 w;
+  if constexpr (sizeof(B) == 8) w = make_uint4((uint32_t)x, (uint32_t)(x >> 32), (uint32_t)x, (uint32_t)(x >> 32));
+  else w = make_uint4(x, x, x, x);
+  uint4* const v = reinterpret_cast<uint4*>(p + head);
+  for (uint32_t i = tid; i < vecs; i += nt) v[i] = w;
+  for (uint32_t i = head + vecs * V + tid; i < len; i += nt) p[i] = x;
 }
 
 template <class T>
@@ -1508,15 +1569,16 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
   unsigned long long sorted = 0ull, moved = 0ull;
   uint32_t jobs = 0u;
   B key[ROWS];
-  auto load = [&](const Bucket& k) {
+  auto fetch = [&](const Bucket& k) {
     if ((k.flags & EQUAL) || k.len > LT) return;
-    load_range<B>(((k.flags & IN_DN) ? dn : d) + k.start, k.len, key);
+    const char* const p = reinterpret_cast<const char*>(((k.flags & IN_DN) ? dn : d) + k.start);
+    for (uint32_t i = tid * 128u; i < k.len * sizeof(B); i += NT * 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
   };
   uint32_t at = blockIdx.x;
   Bucket coming{};
   if (at < nb) {
     coming = plain_n ? Bucket{0ull, plain_n, 0u} : t.bucket[at];
-    load(coming);
+    fetch(coming);
   }
   for (; at < nb; at += gridDim.x) {
     const Bucket bk = coming;
@@ -1544,7 +1606,7 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
         }
       }
       if (same) {
-        for (uint32_t i = tid; i < len; i += NT) dst[i] = x;
+        fill_range<B>(dst, len, x, tid, NT);
         moved += len;
       } else if (tid == 0) {
         const unsigned long long to = atomicAdd(&t.ctl->leftovers, 1ull);
@@ -1552,7 +1614,7 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
         t.left[2 * to + 1] = bk.start + len;
         atomicAdd(&q->left, 1u);
       }
-      if (more) load(coming);
+      if (more) fetch(coming);
       continue;
     }
     sorted += len;
@@ -1560,15 +1622,11 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
 #ifdef GQS_PROFILE
     if (tid == 0) level_note(q, 2u, 2, len);
 #endif
-#pragma unroll
-    for (int j = 0; j < ROWS; ++j) {
-      if ((uint32_t)j * NT >= len) break;
-      key[j] = KeyOps<T>::key(key[j]);
-    }
-    const bool again = sort_range<T>(sm, key, len, dst, [&] {
-      if (more) load(coming);
+    load_range<B>(src, len, key);
+    if (!KeyOps<T>::kIdentity) for_rows<ROWS, NT>(len, [&](int j) { key[j] = KeyOps<T>::key(key[j]); });
+    sort_range<T>(sm, key, len, dst, [&] {
+      if (more) fetch(coming);
     });
-    if (again && more) load(coming);
   }
   if (tid == 0 && (sorted || moved)) {
     atomicAdd(&q->total, sorted + moved);
@@ -1654,7 +1712,7 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
     if (st->eq[b]) {
       if (len <= kCopyChunk) {
         const B x = KeyOps<T>::raw((B)st->value[b]);
-        for (uint32_t i = tid; i < len; i += NT) d[start + i] = x;
+        fill_range<B>(d + start, len, x, tid, NT);
       }
       moved += len;  // longer ones below
       continue;
@@ -1666,11 +1724,7 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
 #endif
     B key[ROWS];
     load_range<B>(area + (size_t)b * LT, len, key);
-#pragma unroll
-    for (int j = 0; j < ROWS; ++j) {
-      if ((uint32_t)j * NT >= len) break;
-      key[j] = KeyOps<T>::key(key[j]);
-    }
+    if (!KeyOps<T>::kIdentity) for_rows<ROWS, NT>(len, [&](int j) { key[j] = KeyOps<T>::key(key[j]); });
     sort_range<T>(sm.local, key, len, d + start, [] {});
   }
   // long ranges of equal keys: every CTA writes a part of each
@@ -1679,7 +1733,7 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
     const B x = KeyOps<T>::raw((B)st->value[b]);
     const uint32_t i0 = (uint32_t)((unsigned long long)len * blockIdx.x / gridDim.x);
     const uint32_t i1 = (uint32_t)((unsigned long long)len * (blockIdx.x + 1u) / gridDim.x);
-    for (uint32_t i = i0 + tid; i < i1; i += NT) d[start + i] = x;
+    fill_range<B>(d + start + i0, i1 - i0, x, tid, NT);
   }
   if (tid == 0 && (sorted || moved)) {
     atomicAdd(&q->total, sorted + moved);
