@@ -21,6 +21,7 @@
 //
 // The reference's counterparts: gqsort_kernel's partition (GPU-Quicksort_OpenCL_1.2/
 // QuicksortKernels.cl:102-240) generalised from one pivot, and lqsort_kernel (267-421).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstddef>
@@ -71,6 +72,7 @@ constexpr uint32_t kMaxSub = 2048;              // cells that those are divided 
 constexpr uint32_t kPartSub = 128;              // and at most so many for one
 constexpr uint32_t kWarpBin = 256;              // longer ones of unequal keys are sorted by a warp each, beyond this by the CTA
 constexpr int kCandidates = 4;
+constexpr uint32_t kCluster = 4;                // CTAs of a small sort that take the sample together
 constexpr uint32_t kCopyChunk = 32768;          // keys of one record of a range of equal keys
 constexpr uint32_t kSmallOver = 10;             // samples a range of a small sort (its ranges have room for three times their mean)
 
@@ -354,6 +356,12 @@ __device__ __forceinline__ uint32_t warp_min<uint32_t>(uint32_t v) { return __re
 template <class B>
 __device__ __forceinline__ B warp_max(B v) { return ~warp_min<B>(~v); }
 
+template <class B>
+__device__ __forceinline__ void prefetch_l2(const B* p, uint32_t len, uint32_t tid, uint32_t nt) {
+  const char* const c = reinterpret_cast<const char*>(p);
+  for (uint32_t i = tid * 128u; i < len * sizeof(B); i += nt * 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(c + i));
+}
+
 // Exclusive scan over the CTA of one value a thread; returns the sum through `total`.
 template <int NT>
 __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* wsum, uint32_t& total) {
@@ -381,11 +389,11 @@ struct MapSmem {
   uint32_t weight[kMaxParts];          // two for each single value in the part
   uint32_t entry[kMaxParts], owner[kMaxParts];  // the part's own cell, and the part that that is in
   uint32_t before[kMaxParts], extra[kMaxParts];  // samples, and weights, in front of it
-  unsigned long long least[kMaxParts], greatest[kMaxParts];
+  uint32_t least[2][kMaxParts], greatest[2][kMaxParts];  // high and low words (32-bit keys: [0])
   uint32_t candidate[kCandidates][kMaxParts];  // indexes of samples
   uint32_t equal[kCandidates][kMaxParts];
   uint32_t cell2[kMaxCells];  // samples per cell by value
-  B wmin[kThreads / 32], wmax[kThreads / 32];
+  B wmin[kCluster * kThreads / 32], wmax[kCluster * kThreads / 32];
   uint32_t wsum[kThreads / 32];
   unsigned long long spread[2][kThreads / 32];
   alignas(16) B sample[1];  // as many as the launch has room for
@@ -394,8 +402,8 @@ constexpr uint32_t kNone = 0xffffu, kWhole = 0xfffeu;  // no part; nor will ther
 
 // Makes the map of src[0, len) for about k ranges: sm.tab and sm.part are its tables, `bins` its ranges (at most bin_room(k));
 // equal(bin, value) is called for each range that holds only keys equal to value. `salt` varies the sample. Every CTA that
-// calls it with the same arguments makes the same map.
-template <class T, class F>
+// calls it with the same arguments makes the same map; the CL CTAs of a cluster read a part of the sample each and hand it round.
+template <class T, uint32_t CL = 1, class F>
 __device__ __forceinline__ void make_map(MapSmem<BOf<T>>& sm, const BOf<T>* src, uint32_t len, uint32_t k, uint32_t salt,
                                          uint32_t over_sample, uint32_t max_sample, KeyMap<T>& map, uint32_t& bins, F&& equal) {
   using B = BOf<T>;
@@ -407,17 +415,31 @@ __device__ __forceinline__ void make_map(MapSmem<BOf<T>>& sm, const BOf<T>* src,
   if (S > len) S = len;
   const uint32_t step = len / S;
   B mn = kmax<B>(), mx = B(0);
-#pragma unroll 8
-  for (uint32_t i = tid; i < S; i += kThreads) {
-    // one key at a pseudo-random place of each of S equal parts
-    uint32_t h = i * 2654435761u + salt * 40503u;
-    h ^= h >> 15;
-    h *= 0x85ebca6bu;
-    const uint32_t at = (uint32_t)(((unsigned long long)i * len) / S) + __umulhi(h, step);
-    const B x = KeyOps<T>::key(src[at]);
-    sm.sample[i] = x;
-    mn = x < mn ? x : mn;
-    mx = x > mx ? x : mx;
+  namespace cg = cooperative_groups;
+  const uint32_t rank = CL > 1u ? cg::this_cluster().block_rank() : 0u;
+  const uint32_t i1 = S * (rank + 1u) / CL;
+  if (CL > 1u) cg::this_cluster().sync();  // the others have started
+  constexpr uint32_t U = CL > 1u ? 4u : 8u;  // loads under way at a time
+  for (uint32_t i0 = S * rank / CL + tid; i0 < i1; i0 += U * kThreads) {
+    B x[U];
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) {
+      // one key at a pseudo-random place of each of S equal parts
+      const uint32_t i = i0 + u * kThreads;
+      uint32_t h = i * 2654435761u + salt * 40503u;
+      h ^= h >> 15;
+      h *= 0x85ebca6bu;
+      if (i < i1) x[u] = KeyOps<T>::key(src[(uint32_t)(((unsigned long long)i * len) / S) + __umulhi(h, step)]);
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) {
+      const uint32_t i = i0 + u * kThreads;
+      if (i >= i1) break;
+#pragma unroll
+      for (uint32_t c = 0; c < CL; ++c) *(CL > 1u ? cg::this_cluster().map_shared_rank(&sm.sample[i], c) : &sm.sample[i]) = x[u];
+      mn = x[u] < mn ? x[u] : mn;
+      mx = x[u] > mx ? x[u] : mx;
+    }
   }
   for (uint32_t i = tid; i < cells; i += kThreads) {
     sm.tab[i] = 0u;
@@ -425,13 +447,22 @@ __device__ __forceinline__ void make_map(MapSmem<BOf<T>>& sm, const BOf<T>* src,
   }
   mn = warp_min<B>(mn);
   mx = warp_max<B>(mx);
-  if (lane == 0) {
-    sm.wmin[warp] = mn;
-    sm.wmax[warp] = mx;
+  if (lane < CL) {
+    const uint32_t at = rank * (kThreads / 32) + warp;
+    *(CL > 1u ? cg::this_cluster().map_shared_rank(&sm.wmin[at], lane) : &sm.wmin[at]) = mn;
+    *(CL > 1u ? cg::this_cluster().map_shared_rank(&sm.wmax[at], lane) : &sm.wmax[at]) = mx;
   }
-  __syncthreads();
-  mn = warp_min<B>(sm.wmin[lane & (kThreads / 32 - 1)]);
-  mx = warp_max<B>(sm.wmax[lane & (kThreads / 32 - 1)]);
+  if (CL > 1u) cg::this_cluster().sync();
+  else __syncthreads();
+  constexpr uint32_t kWarps = CL * kThreads / 32;
+  mn = sm.wmin[lane & (kWarps - 1u)];
+  mx = sm.wmax[lane & (kWarps - 1u)];
+  for (uint32_t i = 32u + lane; i < kWarps; i += 32u) {
+    mn = sm.wmin[i] < mn ? sm.wmin[i] : mn;
+    mx = sm.wmax[i] > mx ? sm.wmax[i] : mx;
+  }
+  mn = warp_min<B>(mn);
+  mx = warp_max<B>(mx);
   // one cell more at each end, for the keys outside the sample's
   map.lo = mn ? mn - 1u : mn;
   const B hi = mx != kmax<B>() ? mx + 1u : mx;
@@ -492,9 +523,13 @@ __device__ __forceinline__ void make_map(MapSmem<BOf<T>>& sm, const BOf<T>* src,
   }
   const bool by_value = kFloating<T> && map.kind;
   __syncthreads();
-  // Cells with the sample of 1.5 ranges and more are divided, and their parts again, twice.
+  // Cells with the sample of 1.5 ranges and more are divided, and their parts again, twice. (A range may end with nearly a whole
+  // cell more than its share: of the words of a pair sort, whose cells are that full more often, one in a few hundred ranges was
+  // longer than kLocal then and cost its sort the persistent kernel, 33 us; theirs are divided from one range's sample on. Other
+  // keys lose by more parts: 1.86 to 1.95 ms for 2^27 f32.)
+  const uint32_t halves = KeyOps<T>::kIdentity && sizeof(B) == 8 && over_sample > kSmallOver ? 2u : 3u;
   constexpr uint32_t R = kMaxCells / kThreads;
-  auto heavy = [&](uint32_t c) { return 2u * c * k >= 3u * S; };
+  auto heavy = [&](uint32_t c) { return 2u * c * k >= halves * S; };
   uint32_t limit[4] = {0u, 0u, 0u, 0u};  // parts made by the end of each round
   uint32_t first = 0u, end = cells, rounds = 0u;
   for (uint32_t round = 0; round < 3u; ++round) {
@@ -523,8 +558,8 @@ __device__ __forceinline__ void make_map(MapSmem<BOf<T>>& sm, const BOf<T>* src,
           sm.part[p].sub = from;
           sm.part[p].mult = from + sub <= last ? sub : 0u;  // 0: no room
           sm.weight[p] = 0u;
-          sm.least[p] = ~0ull;
-          sm.greatest[p] = 0ull;
+          sm.least[0][p] = sm.least[1][p] = ~0u;
+          sm.greatest[0][p] = sm.greatest[1][p] = 0u;
 #pragma unroll
           for (int j = 0; j < kCandidates; ++j) {
             sm.candidate[j][p] = ~0u;
@@ -540,34 +575,52 @@ __device__ __forceinline__ void make_map(MapSmem<BOf<T>>& sm, const BOf<T>* src,
       sm.node[i] = (uint16_t)kNone;
     }
     __syncthreads();
-    // the part of this round that a sample is in, if it is less than kWhole
-    auto part_of = [&](B x) {
-      uint32_t e;
-      if (by_value) e = map.template cell<kFloating<T>>(x);
-      else e = map.template cell<false>(x);
-      uint32_t p = sm.node[e];
-      while (p < n0) p = sm.node[sm.part[p].of(x)];
-      return p;
+    // f(i, x, p) for every sample i, x, that is in a part p of this round; four at a time, each a chain of dependent reads
+    auto in_parts = [&](auto&& f) {
+      for (uint32_t i0 = tid; i0 < S; i0 += 4u * kThreads) {
+        B x[4];
+        uint32_t p[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4u; ++u) {
+          x[u] = sm.sample[i0 + u * kThreads < S ? i0 + u * kThreads : i0];
+          p[u] = sm.node[by_value ? map.template cell<kFloating<T>>(x[u]) : map.template cell<false>(x[u])];
+        }
+        for (uint32_t r = 0; r < round; ++r)
+#pragma unroll
+          for (uint32_t u = 0; u < 4u; ++u)
+            if (p[u] < n0) p[u] = sm.node[sm.part[p[u]].of(x[u])];
+#pragma unroll
+        for (uint32_t u = 0; u < 4u; ++u)
+          if (p[u] < kWhole && i0 + u * kThreads < S) f(i0 + u * kThreads, x[u], p[u]);
+      }
     };
-    for (uint32_t i = tid; i < S; i += kThreads) {
-      const uint32_t p = part_of(sm.sample[i]);
-      if (p >= kWhole) continue;
+    // The atomics are looked at first, as a part of many samples would keep them busy, and of 32 bits: a part's extremes are
+    // found by high words first, then by low words.
+    auto lower = [](uint32_t& m, uint32_t x) {
+      if (x < *(volatile uint32_t*)&m) atomicMin(&m, x);
+    };
+    auto raise = [](uint32_t& m, uint32_t x) {
+      if (x > *(volatile uint32_t*)&m) atomicMax(&m, x);
+    };
+    constexpr int kHigh = sizeof(B) == 8 ? 32 : 0;
+    in_parts([&](uint32_t i, B x, uint32_t p) {
       // the first samples of four parts of the sample: a frequent value most likely
-      atomicMin(&sm.candidate[i / kThreads % kCandidates][p], i);
-      atomicMin(&sm.least[p], (unsigned long long)sm.sample[i]);
-      atomicMax(&sm.greatest[p], (unsigned long long)sm.sample[i]);
-    }
+      lower(sm.candidate[i / kThreads % kCandidates][p], i);
+      lower(sm.least[0][p], (uint32_t)(x >> kHigh));
+      raise(sm.greatest[0][p], (uint32_t)(x >> kHigh));
+    });
     __syncthreads();
-    for (uint32_t i = tid; i < S; i += kThreads) {
-      const B x = sm.sample[i];
-      const uint32_t p = part_of(x);
-      if (p >= kWhole) continue;
+    in_parts([&](uint32_t, B x, uint32_t p) {
 #pragma unroll
       for (int j = 0; j < kCandidates; ++j)
         if (sm.candidate[j][p] != ~0u && x == sm.sample[sm.candidate[j][p]]) atomicAdd(&sm.equal[j][p], 1u);
-    }
+      if (sizeof(B) == 8) {
+        if ((uint32_t)(x >> kHigh) == sm.least[0][p]) lower(sm.least[1][p], (uint32_t)x);
+        if ((uint32_t)(x >> kHigh) == sm.greatest[0][p]) raise(sm.greatest[1][p], (uint32_t)x);
+      }
+    });
     __syncthreads();
-    for (uint32_t p = n0 + tid; p < n1; p += kThreads) {
+    for (uint32_t p = n0 + warp; p < n1; p += kThreads / 32) {
       Part<B> part = sm.part[p];
       const uint32_t e = sm.entry[p], sub = part.mult;
       if (!sub) continue;
@@ -580,31 +633,34 @@ __device__ __forceinline__ void make_map(MapSmem<BOf<T>>& sm, const BOf<T>* src,
         }
       if ((sm.tab[e] - most) * k <= S) {  // the others are a range at most
         part.mult = 0u;
-        sm.weight[p] = 2u;
-        sm.node[part.sub + 1u] = (uint16_t)kWhole;
+        if (lane == 0) {
+          sm.weight[p] = 2u;
+          sm.node[part.sub + 1u] = (uint16_t)kWhole;
+        }
       } else {
-        part.lo = (B)sm.least[p];
-        part.span = (B)sm.greatest[p] - part.lo;
+        auto whole = [&](const uint32_t (&w)[2][kMaxParts]) { return sizeof(B) == 8 ? (B)w[0][p] << kHigh | w[1][p] : (B)w[0][p]; };
+        part.lo = whole(sm.least);
+        part.span = whole(sm.greatest) - part.lo;
         const int bits = bits_of(part.span);
         part.right = bits > 32 ? (uint32_t)bits - 32u : 0u;
         part.left = bits < 32 ? 32u - (uint32_t)bits : 0u;
         const unsigned long long top = (unsigned long long)((uint32_t)(part.span >> part.right) << part.left) + 1ull;
         part.mult = (uint32_t)(((unsigned long long)sub << 32) / top);
       }
-      sm.part[p] = part;
       // the part that this one's cell is in: the last of the round before whose cells start at or before it
-      uint32_t o = kNone;
+      uint32_t o = 0u;
       if (round)
-        for (uint32_t j = limit[round - 1u]; j < n0; ++j)
-          if (sm.node[sm.entry[j]] == j && sm.part[j].sub <= e) o = j;
-      sm.owner[p] = o;
+        for (uint32_t j = limit[round - 1u] + lane; j < n0; j += 32u)
+          if (sm.node[sm.entry[j]] == j && sm.part[j].sub <= e) o = j + 1u;
+      o = __reduce_max_sync(0xffffffffu, o);
+      __syncwarp();
+      if (lane == 0) {
+        sm.part[p] = part;
+        sm.owner[p] = o ? o - 1u : kNone;
+      }
     }
     __syncthreads();
-    for (uint32_t i = tid; i < S; i += kThreads) {
-      const B x = sm.sample[i];
-      const uint32_t p = part_of(x);
-      if (p < kWhole) atomicAdd(&sm.tab[sm.part[p].of(x)], 1u);
-    }
+    in_parts([&](uint32_t, B x, uint32_t p) { atomicAdd(&sm.tab[sm.part[p].of(x)], 1u); });
     __syncthreads();
     first = end;
     end = last;
@@ -659,19 +715,27 @@ __device__ __forceinline__ void make_map(MapSmem<BOf<T>>& sm, const BOf<T>* src,
       }
     for (uint32_t round = 0; round < rounds; ++round) {
       __syncthreads();
-      for (uint32_t p = limit[round] + tid; p < limit[round + 1u]; p += kThreads) {
+      for (uint32_t p = limit[round] + warp; p < limit[round + 1u]; p += kThreads / 32) {  // its cells 32 at a time
         if (sm.tab[sm.entry[p]] != (0x80000000u | p)) continue;
-        const Part<B>& part = sm.part[p];
+        const Part<B> part = sm.part[p];
         uint32_t in_front = sm.before[p] | (sm.extra[p] << 16);
         const uint32_t sub = part.mult ? part.of(kmax<B>()) - part.sub + 1u : 3u;
-        for (uint32_t i = 0; i < sub; ++i) {
-          const uint32_t e = part.sub + i, c = sum_of(e);
-          settle(e, in_front & 0xffffu, in_front >> 16);
+        for (uint32_t i0 = 0; i0 < sub; i0 += 32u) {
+          const uint32_t i = i0 + lane, e = part.sub + i;
+          const uint32_t c = i < sub ? sum_of(e) + (part.mult || i >= 2u ? 0u : 1u << 16) : 0u;
+          uint32_t inc = c;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+            if ((int)lane >= o) inc += u;
+          }
+          const uint32_t front = in_front + inc - c;
+          if (i < sub) settle(e, front & 0xffffu, front >> 16);
           if (!part.mult && i == 1u) {
             equal(sm.tab[e], part.lo);
             sm.tab[e] |= kEqual;
           }
-          in_front += c + (part.mult || i == 2u ? 0u : 1u << 16);
+          in_front += __shfl_sync(0xffffffffu, inc, 31);
         }
       }
     }
@@ -1105,8 +1169,8 @@ union SmallSmem {
   } s;
 };
 
-template <class T>
-__global__ void __launch_bounds__(kThreads, SP_MINB) split_small(const BOf<T>* src, BOf<T>* area, uint32_t n, uint32_t k, Small* st, uint32_t tile_keys,
+template <class T, uint32_t CL>
+__global__ void __cluster_dims__(CL) __launch_bounds__(kThreads, SP_MINB) split_small(const BOf<T>* src, BOf<T>* area, uint32_t n, uint32_t k, Small* st, uint32_t tile_keys,
                                                                  Queue* q) {
   using B = BOf<T>;
   constexpr int ROWS = Sizes<B>::kTileRows;
@@ -1119,11 +1183,14 @@ __global__ void __launch_bounds__(kThreads, SP_MINB) split_small(const BOf<T>* s
   const uint32_t tiles = (n + tile_keys - 1u) / tile_keys;
   KeyMap<T> map;
   uint32_t bins;
-  if (blockIdx.x == 0) {
-    clear(q, sizeof(Queue));
-    clear(st->eq, bin_room(k) * 4);
+  if (blockIdx.x < tiles) {  // read while the map is made
+    const uint32_t k0 = blockIdx.x * tile_keys, here = n - k0 < tile_keys ? n - k0 : tile_keys;
+    prefetch_l2(src + k0, here, tid, kThreads);
   }
-  make_map<T>(sm.map, src, n, k, 0u, kSmallOver, Sizes<B>::kSmallSample, map, bins, [&](uint32_t b, B x) {
+  // (there are two tiles at least, so there is a CTA 1)
+  if (blockIdx.x == 0) clear(st->eq, bin_room(k) * 4);
+  if (blockIdx.x == 1) clear(q, sizeof(Queue));
+  make_map<T, CL>(sm.map, src, n, k, 0u, kSmallOver, Sizes<B>::kSmallSample, map, bins, [&](uint32_t b, B x) {
     if (blockIdx.x == 0) {
       st->eq[b] = 1u;
       st->value[b] = x;
@@ -1132,6 +1199,8 @@ __global__ void __launch_bounds__(kThreads, SP_MINB) split_small(const BOf<T>* s
   if (blockIdx.x == 0 && tid == 0) {
     st->bins = bins;
     st->left = 0ull;
+  }
+  if (blockIdx.x == 1 && tid == 0) {
     q->part_keys = n;
     q->part_jobs = 1u;
     q->chunks = tiles;
@@ -1257,6 +1326,29 @@ __device__ __forceinline__ void for_rows(uint32_t len, F&& f) {
   }
 }
 
+// The keys of a range while it is sorted: less its least, mn. The words of a pair sort are a key above a value, and the values
+// seldom fill their 32 bits: the bits that no value of the range has are left out, so that equal steps of the result do not leave
+// the bins between two keys empty.
+template <class T>
+struct Near {
+  using B = BOf<T>;
+  static constexpr bool kWords = KeyOps<T>::kIdentity && sizeof(B) == 8;
+  B mn;
+  uint32_t width;  // of the values
+  __device__ __forceinline__ B in(B x) const {
+    if constexpr (kWords) return (((x >> 32) - (mn >> 32)) << width | (uint32_t)x) - (uint32_t)mn;
+    else return x - mn;
+  }
+  __device__ __forceinline__ B out(B y) const {
+    if constexpr (kWords) {
+      y += (uint32_t)mn;
+      return ((y >> width) + (mn >> 32)) << 32 | (y & ((B(1) << width) - 1u));
+    } else {
+      return y + mn;
+    }
+  }
+};
+
 // How a range's keys (less its least, mn) fall into bins: equal steps of the integer, or of the value.
 template <class T>
 struct BinMap {
@@ -1265,8 +1357,8 @@ struct BinMap {
   uint32_t bins, sh, mult;  // (x >> sh) * mult / 2^32, or x itself (mult 0)
   float flo, scale;
   bool by_value;
-  __device__ __forceinline__ BinMap(B lo, B hi, uint32_t n, bool first) : mn(lo), bins(n), flo(0.f), scale(0.f), by_value(false) {
-    const B range = hi - lo;
+  // `range`: hi, less lo. `key`: one of the range's keys, if `has`.
+  __device__ __forceinline__ BinMap(B lo, B hi, B range, uint32_t n, bool first, B key, bool has) : mn(lo), bins(n), flo(0.f), scale(0.f), by_value(false) {
     const int over = bits_of(range) - 32;
     sh = over > 0 ? (uint32_t)over : 0u;
     const uint32_t top = (uint32_t)(range >> sh);
@@ -1281,6 +1373,15 @@ struct BinMap {
         const float b = as_float<T>(hi), w = __fsub_rn(b, flo);
         scale = __fdiv_rn((float)bins * 0.99999f, w);
         by_value = finite_span(flo, b, w) && scale < 3e38f;
+        if (by_value) {
+          // the one that has nearer to a half of these keys in the middle half of its bins
+          auto off = [&](uint32_t bin) {
+            const int in = __syncthreads_count(has && bin >= n / 4u && bin < n / 4u * 3u);
+            return 2 * in;
+          };
+          const int all = __syncthreads_count(has);
+          by_value = abs(off(of<true>(key - lo)) - all) <= abs(off(of<false>(key - lo)) - all);
+        }
       }
     }
   }
@@ -1314,16 +1415,20 @@ __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[S
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   dst += off;
   B mn = kmax<B>(), mx = B(0);
+  uint32_t values = 0u;
   for_rows<ROWS, NT>(len, [&](int j) {
     mn = key[j] < mn ? key[j] : mn;
     mx = key[j] > mx ? key[j] : mx;
+    if (Near<T>::kWords) values |= (uint32_t)key[j];
   });
   mn = warp_min<B>(mn);
   mx = warp_max<B>(mx);
+  if (Near<T>::kWords) values = __reduce_or_sync(0xffffffffu, values);
   __syncthreads();  // the range before has left shared memory
   if (lane == 0) {
     sm.wmin[warp] = mn;
     sm.wmax[warp] = mx;
+    if (Near<T>::kWords) sm.wsum[warp] = values;
   }
   // bins: a power of two, at least as many as keys
   constexpr uint32_t kMinBins = 8u * NT < LT ? 8u * NT : LT;
@@ -1337,10 +1442,12 @@ __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[S
   __syncthreads();
   mn = warp_min<B>(sm.wmin[lane & (NT / 32 - 1)]);
   mx = warp_max<B>(sm.wmax[lane & (NT / 32 - 1)]);
-  const BinMap<T> map(mn, mx, bins, first);
+  Near<T> near{mn, 0u};
+  if (Near<T>::kWords) near.width = (uint32_t)bits_of(__reduce_or_sync(0xffffffffu, sm.wsum[lane & (NT / 32 - 1)]));
+  const BinMap<T> map(mn, mx, near.in(mx), bins, first, key[0], tid < len);
   auto count = [&]<bool VALUE>() {
     for_rows<ROWS, NT>(len, [&](int j) {
-      key[j] -= mn;
+      key[j] = near.in(key[j]);
       const uint32_t b = map.template of<VALUE>(key[j]);
       atomicAdd(&sm.cur[b >> 1], b & 1u ? 0x10000u : 1u);
     });
@@ -1482,7 +1589,7 @@ __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[S
   const B* const mine = &sm.keys[S::slot(tid)];
   static_assert(NT % 128u == 0u, "slot(i + NT) is slot(i) + NT");
   B* const to = dst + tid;
-  for_rows<ROWS, NT>(len, [&](int j) { to[j * NT] = KeyOps<T>::raw(mine[j * NT] + mn); });
+  for_rows<ROWS, NT>(len, [&](int j) { to[j * NT] = KeyOps<T>::raw(near.out(mine[j * NT])); });
 }
 
 // v = *p where `use`: as inline code, so that the loads stay one behind the other with nothing between them.
@@ -1571,8 +1678,7 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
   B key[ROWS];
   auto fetch = [&](const Bucket& k) {
     if ((k.flags & EQUAL) || k.len > LT) return;
-    const char* const p = reinterpret_cast<const char*>(((k.flags & IN_DN) ? dn : d) + k.start);
-    for (uint32_t i = tid * 128u; i < k.len * sizeof(B); i += NT * 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
+    prefetch_l2(((k.flags & IN_DN) ? dn : d) + k.start, k.len, tid, NT);
   };
   uint32_t at = blockIdx.x;
   Bucket coming{};
@@ -1640,7 +1746,7 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
 
 constexpr uint32_t kOwnRanges = 32;  // of one CTA of local_small
 struct Extent {
-  uint32_t bin, start, len;
+  uint32_t bin, start, len, equal;
 };
 template <class B>
 struct SmallSortSmem {
@@ -1651,10 +1757,14 @@ struct SmallSortSmem {
   Extent fill[Sizes<B>::kSmallMax / kCopyChunk + 1];  // long ranges of equal keys
 };
 
-// Every CTA of local_small calls this when it has read the cursors; the last one zeroes them.
-__device__ __forceinline__ void leave_small(Small* st, uint32_t bins) {
+// Every CTA of local_small takes a turn when it has read the cursors; the last one zeroes them, as its last work, so that no CTA
+// waits for its turn's answer.
+__device__ __forceinline__ uint32_t take_turn(Small* st) {
   __threadfence();
-  if (__syncthreads_or(threadIdx.x == 0 && atomicAdd(&st->done, 1u) == gridDim.x - 1u)) {
+  return atomicAdd(&st->done, 1u);
+}
+__device__ __forceinline__ void leave_small(Small* st, uint32_t bins, uint32_t turn) {  // thread 0's turn
+  if (__syncthreads_or(threadIdx.x == 0 && turn == gridDim.x - 1u)) {
     for (uint32_t i = threadIdx.x; i < bins; i += blockDim.x) st->cursor[i] = 0u;
     if (threadIdx.x == 0) st->done = 0u;
   }
@@ -1674,33 +1784,42 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
   pdl_trigger();
   const uint32_t bins = st->bins;
   uint32_t c[R], sum = 0u, total;
-  bool full = false;  // a range ran out of room
+  uint32_t equal = 0u;  // bit i: c[i] is of a range of equal keys, to be written by this CTA
+  bool full = false;    // a range ran out of room
+  const uint32_t per = (bins + NT - 1u) / NT;
   if (tid == 0) sm.fills = 0u;
-  __syncthreads();
 #pragma unroll
   for (uint32_t i = 0; i < R; ++i) {
-    const uint32_t b = tid * R + i;
-    c[i] = b < bins ? st->cursor[b] : 0u;
-    if (c[i] > LT && !st->eq[b]) full = true;
+    const uint32_t b = tid * per + i;
+    c[i] = 0u;
+    if (i < per && b < bins) {
+      c[i] = st->cursor[b];
+      if (b % gridDim.x == blockIdx.x && st->eq[b]) equal |= 1u << i;
+    }
+  }
+#pragma unroll
+  for (uint32_t i = 0; i < R; ++i) {
+    if (c[i] > LT && !st->eq[tid * per + i]) full = true;
     sum += c[i];
   }
-  if (__syncthreads_or(full)) {
+  full = __syncthreads_or(full);  // (and every thread has its counts)
+  const uint32_t turn = tid == 0 ? take_turn(st) : 0u;
+  if (full) {
     if (blockIdx.x == 0 && tid == 0) {  // d is as it was: all of it is left to the persistent kernel
       st->table[0] = 0ull;
       st->table[1] = n;
       st->left = 1ull;
       q->left = 1u;
     }
-    leave_small(st, bins);
+    leave_small(st, bins, turn);
     return;
   }
-  leave_small(st, bins);
   uint32_t at = block_scan<NT>(sum, sm.wsum, total);
 #pragma unroll
   for (uint32_t i = 0; i < R; ++i) {
-    const uint32_t b = tid * R + i;
-    if (b < bins && b % gridDim.x == blockIdx.x) sm.own[b / gridDim.x] = Extent{b, at, c[i]};
-    if (c[i] > kCopyChunk) sm.fill[atomicAdd(&sm.fills, 1u)] = Extent{b, at, c[i]};
+    const uint32_t b = tid * per + i;
+    if (i < per && b < bins && b % gridDim.x == blockIdx.x) sm.own[b / gridDim.x] = Extent{b, at, c[i], equal >> i & 1u};
+    if (c[i] > kCopyChunk) sm.fill[atomicAdd(&sm.fills, 1u)] = Extent{b, at, c[i], 1u};
     at += c[i];
   }
   __syncthreads();
@@ -1709,7 +1828,7 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
   for (uint32_t o = 0; o * gridDim.x + blockIdx.x < bins; ++o) {
     const uint32_t b = sm.own[o].bin, start = sm.own[o].start, len = sm.own[o].len;
     if (!len || !GQS_OK(start + len <= n, q, 0xD202ull)) continue;
-    if (st->eq[b]) {
+    if (sm.own[o].equal) {
       if (len <= kCopyChunk) {
         const B x = KeyOps<T>::raw((B)st->value[b]);
         fill_range<B>(d + start, len, x, tid, NT);
@@ -1735,6 +1854,7 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
     const uint32_t i1 = (uint32_t)((unsigned long long)len * (blockIdx.x + 1u) / gridDim.x);
     fill_range<B>(d + start + i0, i1 - i0, x, tid, NT);
   }
+  leave_small(st, bins, turn);
   if (tid == 0 && (sorted || moved)) {
     atomicAdd(&q->total, sorted + moved);
     atomicAdd(&q->done, sorted + moved);
@@ -1822,7 +1942,8 @@ cudaError_t launch_t(const SplitArgs& a, SplitResult* out) {
   static const cudaError_t attr = [] {
     cudaError_t e = allow_smem(split_scatter<T>, sizeof(ScatterSmem<B>));
     if (e == cudaSuccess) e = allow_smem(split_map<T>, sizeof(MapSmem<B>) + Sizes<B>::kMaxSample * sizeof(B));
-    if (e == cudaSuccess) e = allow_smem(split_small<T>, sizeof(SmallSmem<B>));
+    if (e == cudaSuccess) e = allow_smem(split_small<T, 1>, sizeof(SmallSmem<B>));
+    if (e == cudaSuccess) e = allow_smem(split_small<T, kCluster>, sizeof(SmallSmem<B>));
     if (e == cudaSuccess) e = allow_smem(local_sort<T>, sizeof(LocalSmem<B>));
     if (e == cudaSuccess) e = allow_smem(local_small<T>, sizeof(SmallSortSmem<B>));
     return e;
@@ -1850,7 +1971,13 @@ cudaError_t launch_t(const SplitArgs& a, SplitResult* out) {
     Small* st = reinterpret_cast<Small*>(base + lay.small_at);
     B* area = reinterpret_cast<B*>(base + lay.area_at);
     const uint32_t n = (uint32_t)a.n, tiles = (n + tile_keys - 1u) / tile_keys, k = small_count<B>(a.n, a.sms);
-    go(split_small<T>, least(sms * SP_MINB, tiles), kThreads, sizeof(SmallSmem<B>), (const B*)d, area, n, k, st, tile_keys, a.q);
+    // CTAs that read the sample each keep L2 busy once every SM has two of them; a cluster's CTAs share SMs where others are idle
+    if (tiles > sms) {
+      const uint32_t ctas = (least(sms * SP_MINB, tiles) + kCluster - 1u) / kCluster * kCluster;
+      go(split_small<T, kCluster>, ctas, kThreads, sizeof(SmallSmem<B>), (const B*)d, area, n, k, st, tile_keys, a.q);
+    } else {
+      go(split_small<T, 1>, tiles, kThreads, sizeof(SmallSmem<B>), (const B*)d, area, n, k, st, tile_keys, a.q);
+    }
     const uint32_t ranges = bin_room(k), few = sms * Sizes<B>::kSortCtas, enough = (ranges + kOwnRanges - 1u) / kOwnRanges;
     go(local_small<T>, few > ranges ? ranges : few > enough ? few : enough, Sizes<B>::kSortThreads, sizeof(SmallSortSmem<B>), d, (const B*)area, n, st, a.q);
     out->table = reinterpret_cast<const unsigned long long*>(base + lay.small_at + offsetof(Small, table));
