@@ -757,10 +757,14 @@ gqs_status gqs_reserve(gqs_ctx* c, int dtype, size_t n, size_t nseg, int with_bu
   if (n >= (1ull << 40) || nseg >= (1ull << 31)) return GQS_ERR_INVALID;
   // the split has scratch of its own, and may leave ranges that become segments
   const size_t nseg_in = nseg ? nseg : 1;
-  if (use_split(c, dtype, n, nseg <= 1)) {
-    gqs_status st = grow_split(c, gqs::split_scratch_bytes(dtype, n, nseg_in, nseg <= 1, c->num_sms));
+  const size_t reach = c->auto_variant[dtype] || nseg_in > 1 ? (1ull << 31) - 1 : 1ull << 21;  // the largest that use_split takes
+  const size_t m = std::min(n, reach);
+  if (use_split(c, dtype, m, nseg_in == 1)) {
+    size_t bytes = gqs::split_scratch_bytes(dtype, m, 1, true, c->num_sms);
+    if (nseg_in > 1) bytes = std::max(bytes, gqs::split_scratch_bytes(dtype, m, nseg_in, false, c->num_sms));
+    gqs_status st = grow_split(c, bytes);
     if (st != GQS_OK) return st;
-    nseg = std::max(nseg_in, n / 4096 + 1);
+    nseg = std::max(nseg_in, m / 4096 + 1);
   }
   const size_t cap = job_capacity(vi, n, nseg ? nseg : 1);
   if (cap >= (1ull << 32) || ticket_ring(vi, n, nseg ? nseg : 1) > (1ull << 31)) return GQS_ERR_INVALID;

@@ -2024,7 +2024,13 @@ cudaError_t launch_t(const SplitArgs& a, SplitResult* out) {
 }  // namespace
 
 size_t split_scratch_bytes(int dtype, size_t n, size_t nseg, bool plain, int sms) {
-  return kDtypeBytes(dtype) == 4 ? Layout<uint32_t>(n, nseg, plain, sms).bytes : Layout<uint64_t>(n, nseg, plain, sms).bytes;
+  auto bytes = [&]<class B>() {
+    // never less than a smaller plain sort takes: the roomy ranges of the longest small one need more than somewhat longer sorts
+    const size_t all = Layout<B>(n, nseg, plain, sms).bytes, most = Sizes<B>::kSmallMax;
+    const size_t small = plain && n > most ? Layout<B>(most, 1, true, sms).bytes : 0;
+    return all > small ? all : small;
+  };
+  return kDtypeBytes(dtype) == 4 ? bytes.template operator()<uint32_t>() : bytes.template operator()<uint64_t>();
 }
 
 size_t split_clear_bytes() { return sizeof(Small); }
