@@ -322,13 +322,18 @@ struct KeyMap {
       return (uint32_t)(offset(key) >> sh);
     }
   }
-  template <bool VALUE, bool PARTS_>
-  __device__ __forceinline__ uint32_t bin(B key, const uint32_t* tab, const Part<B>* part) const {
+  // (tables of short() entries take the mark of a part and kEqual from the two highest bits)
+  template <bool VALUE, bool PARTS_, class E>
+  __device__ __forceinline__ uint32_t bin(B key, const E* tab, const Part<B>* part) const {
+    constexpr int kTop = sizeof(E) * 8 - 1;
     uint32_t e = tab[cell<VALUE>(key)];
-    if constexpr (PARTS_)
-      while (e >> 31) e = tab[part[e & 0x7fffffffu].of(key)];
+    if constexpr (PARTS_) {
+      while (e >> kTop) e = tab[part[e & ((1u << kTop) - 1u)].of(key)];
+      if (sizeof(E) == 2 && e >> 14) e ^= 1u << 14 ^ kEqual;
+    }
     return e;
   }
+  static __device__ __forceinline__ uint16_t narrow(uint32_t e) { return (uint16_t)((e & 0x3fffu) | (e >> 16 & 0xc000u)); }
 };
 // Calls f.template operator()<VALUE, PARTS_>() with what `kind` says.
 template <class T, class F>
@@ -970,49 +975,59 @@ struct TileSmem {
 // count), groups the keys by range in shared memory, calls between(), then puts each key with put(range, first, key, index):
 // the tile's part of the range is key indexes [.., ..) of the groups and starts at `first` - index of its first.
 // The reservation's round trip to L2 is hidden behind the grouping, the next tile's loads (between) behind the writes.
-template <class T, bool VALUE, bool PARTS_, bool COUNT_EQUAL, class Reserve, class Between, class Put>
-__device__ __forceinline__ void scatter_tile(TileSmem<BOf<T>>& sm, const KeyMap<T>& map, const uint32_t* tab, const Part<BOf<T>>* part,
+template <class T, bool VALUE, bool PARTS_, bool COUNT_EQUAL, class E, class Reserve, class Between, class Put>
+__device__ __forceinline__ void scatter_tile(TileSmem<BOf<T>>& sm, const KeyMap<T>& map, const E* tab, const Part<BOf<T>>* part,
                                              uint32_t bins, const BOf<T> (&key)[Sizes<BOf<T>>::kTileRows], uint32_t here,
                                              Reserve&& reserve, Between&& between, Put&& put) {
   using B = BOf<T>;
   constexpr int ROWS = Sizes<B>::kTileRows;
   const uint32_t tid = threadIdx.x, lane = tid & 31u;
-  uint32_t at[ROWS];  // (range << 16) | place in the tile's part of it; kLeft: left out
-  constexpr uint32_t kLeft = ~0u;
+  // Without parts: the keys' ranges, two in a word, and a second atomic for their places, once the counters hold the ranges' starts.
+  // With parts, where hot counters make atomics slow: (range << 16) | place in the tile's part of it. kLeft: not moved.
+  uint32_t at[PARTS_ ? ROWS : ROWS / 2] = {};
+  constexpr uint32_t kLeft = PARTS_ ? ~0u : 0xffffu;
+  auto range_of = [&](int j) { return j & 1 ? at[j / 2] >> 16 : at[j / 2] & 0xffffu; };
+  auto same_row = [&](uint32_t b) { return __all_sync(0xffffffffu, b == __shfl_sync(0xffffffffu, b, 0)); };
   const bool full = !PARTS_ && here == (uint32_t)ROWS * kThreads;
   uint32_t moved = here;
-  if (full) {
-#pragma unroll
-    for (int j = 0; j < ROWS; ++j) at[j] = map.template bin<VALUE, PARTS_>(key[j], tab, part);
-    // 32 adds to one counter run one by one: where rows seem to be of one range each, one add a row
-    const bool runs = __all_sync(0xffffffffu, at[0] == __shfl_sync(0xffffffffu, at[0], 0)) ||
-                      __all_sync(0xffffffffu, at[ROWS / 2] == __shfl_sync(0xffffffffu, at[ROWS / 2], 0));
-    if (!runs) {
-#pragma unroll
-      for (int j = 0; j < ROWS; ++j) at[j] = (at[j] << 16) | atomicAdd(&sm.cnt[at[j]], 1u);
-    } else {
-#pragma unroll
-      for (int j = 0; j < ROWS; ++j) {
-        const uint32_t b = at[j];
-        uint32_t rank = 0u;
-        if (__all_sync(0xffffffffu, b == __shfl_sync(0xffffffffu, b, 0))) {
-          if (lane == 0) rank = atomicAdd(&sm.cnt[b], 32u);
-          rank = __shfl_sync(0xffffffffu, rank, 0) + lane;
-        } else {
-          rank = atomicAdd(&sm.cnt[b], 1u);
-        }
-        at[j] = (b << 16) | rank;
-      }
-    }
-  } else {
+  bool runs = false;
+  if constexpr (PARTS_) {
 #pragma unroll
     for (int j = 0; j < ROWS; ++j) {
       at[j] = kLeft;
       if ((uint32_t)j * kThreads + tid < here) {
         const uint32_t b = map.template bin<VALUE, PARTS_>(key[j], tab, part);
-        if (!PARTS_ || b < kEqual) at[j] = (b << 16) | atomicAdd(&sm.cnt[b], 1u);
+        if (b < kEqual) at[j] = (b << 16) | atomicAdd(&sm.cnt[b], 1u);
         else if (COUNT_EQUAL) atomicAdd(&sm.cnt[b & kBinMask], 1u << 16);
       }
+    }
+  } else if (full) {
+#pragma unroll
+    for (int j = 0; j < ROWS; j += 2)
+      at[j / 2] = map.template bin<VALUE, PARTS_>(key[j], tab, part) | map.template bin<VALUE, PARTS_>(key[j + 1], tab, part) << 16;
+    // 32 adds to one counter run one by one: where rows seem to be of one range each, one add a row
+    const bool r0 = same_row(range_of(0)), r1 = same_row(range_of(ROWS / 2));
+    runs = r0 || r1;
+    if (!runs) {
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j) atomicAdd(&sm.cnt[range_of(j)], 1u);
+    } else {
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j) {
+        const uint32_t b = range_of(j);
+        if (!same_row(b)) atomicAdd(&sm.cnt[b], 1u);
+        else if (lane == 0) atomicAdd(&sm.cnt[b], 32u);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+      uint32_t b = kLeft;
+      if ((uint32_t)j * kThreads + tid < here) {
+        b = map.template bin<VALUE, PARTS_>(key[j], tab, part);
+        atomicAdd(&sm.cnt[b], 1u);
+      }
+      at[j / 2] |= b << 16 * (j & 1);
     }
   }
   __syncthreads();
@@ -1040,17 +1055,34 @@ __device__ __forceinline__ void scatter_tile(TileSmem<BOf<T>>& sm, const KeyMap<
       }
   }
   __syncthreads();
-  if (full) {
-#pragma unroll
-    for (int j = 0; j < ROWS; ++j) sm.keys[sm.cnt[at[j] >> 16] + (at[j] & 0xffffu)] = key[j];
-  } else {
+  if constexpr (PARTS_) {
 #pragma unroll
     for (int j = 0; j < ROWS; ++j)
       if (at[j] != kLeft) {
         const uint32_t i = sm.cnt[at[j] >> 16] + (at[j] & 0xffffu);
         sm.keys[i] = key[j];
-        if (PARTS_) sm.bin[i] = (uint16_t)(at[j] >> 16);  // cheaper than to find it again
+        sm.bin[i] = (uint16_t)(at[j] >> 16);  // cheaper than to find it again
       }
+  } else if (full && !runs) {
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) sm.keys[atomicAdd(&sm.cnt[range_of(j)], 1u)] = key[j];
+  } else if (full) {
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+      const uint32_t b = range_of(j);
+      uint32_t i = 0u;
+      if (!same_row(b)) {
+        i = atomicAdd(&sm.cnt[b], 1u);
+      } else {
+        if (lane == 0) i = atomicAdd(&sm.cnt[b], 32u);
+        i = __shfl_sync(0xffffffffu, i, 0) + lane;
+      }
+      sm.keys[i] = key[j];
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j)
+      if (range_of(j) != kLeft) sm.keys[atomicAdd(&sm.cnt[range_of(j)], 1u)] = key[j];
   }
   if (b0 < bins) sm.gbase[b0] = base0 - ex0;
   between();
@@ -1072,7 +1104,7 @@ __device__ __forceinline__ void scatter_tile(TileSmem<BOf<T>>& sm, const KeyMap<
 template <class B>
 struct ScatterSmem {
   TileSmem<B> tile;
-  uint32_t tab[kMaxCells + kMaxSub];
+  uint16_t tab[kMaxCells + kMaxSub];
   Part<B> part[kMaxParts];
 };
 
@@ -1136,7 +1168,7 @@ __global__ void __launch_bounds__(kThreads, SP_MINB) split_scatter(const BOf<T>*
       out = dst + start;
       const uint32_t* const cell = v.cell + r->cell0;
       __syncthreads();
-      for (uint32_t i = tid; i < map.used; i += kThreads) sm.tab[i] = cell[i];
+      for (uint32_t i = tid; i < map.used; i += kThreads) sm.tab[i] = KeyMap<T>::narrow(cell[i]);
       for (uint32_t i = tid; i < (map.kind & PART_COUNT); i += kThreads) sm.part[i] = static_cast<const Part<B>*>(v.part)[r->bin0 / 4u + i];
     }
     if (!bins) {  // equal keys only, which need not move
