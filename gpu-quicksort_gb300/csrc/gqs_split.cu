@@ -12,7 +12,9 @@
 //   local_sort     every range sorted in shared memory, into d
 // Plain sorts of at most kSmallMax keys take two kernels instead: split_small (every CTA makes the
 // map for itself, then scatters into ranges with room for kLocal keys each, so that nothing is
-// counted first) and local_sort over those ranges.
+// counted first) and local_small over those ranges.
+// Device time against the persistent kernel's binary levels, which took these sorts before: 2^28 u32 10.7 to 3.10 ms, 2^26 f64
+// 5.05 to 1.86 ms, 2^20 u32 84 to 27 us (that was with a split of its own in front).
 // The order of keys inside a range does not matter to the next step, so a key's place in it
 // is the old value of a counter (one shared-memory atomic), not a stable rank.
 //
@@ -36,34 +38,8 @@ namespace {
 template <class T>
 using BOf = typename KeyOps<T>::B;
 
-#ifndef SP_KPT32
-#define SP_KPT32 16
-#endif
-#ifndef SP_MINB
-#define SP_MINB 2
-#endif
-#ifndef LS_NT32
-#define LS_NT32 256
-#endif
-#ifndef LS_MINB32
-#define LS_MINB32 3
-#endif
-#ifndef LS_LT32
-#define LS_LT32 8192
-#endif
-#ifndef LS_NT64
-#define LS_NT64 256
-#endif
-#ifndef LS_MINB64
-#define LS_MINB64 3
-#endif
-#ifndef LS_LT64
-#define LS_LT64 4096
-#endif
-#ifndef SP_OVER
-#define SP_OVER 32
-#endif
-constexpr int kThreads = 512;
+constexpr int kThreads = 512;                   // of the map, count and scatter kernels
+constexpr uint32_t kTileCtas = 2;               // of the scatter kernels on an SM: three spill their keys (2^28 u32: 3.10 to 3.66 ms)
 constexpr uint32_t kMaxBins = 1024;             // ranges one segment is split into (bin_room: the map may make more)
 constexpr uint32_t kBinSlots = 2564;            // bin_room(kMaxBins)
 constexpr uint32_t kMaxCells = 4096;
@@ -72,16 +48,19 @@ constexpr uint32_t kMaxSub = 2048;              // cells that those are divided 
 constexpr uint32_t kPartSub = 128;              // and at most so many for one
 constexpr uint32_t kWarpBin = 256;              // longer ones of unequal keys are sorted by a warp each, beyond this by the CTA
 constexpr int kCandidates = 4;
+constexpr uint32_t kOver = 32;                  // samples a range of a counted level
 constexpr uint32_t kCluster = 4;                // CTAs of a small sort that take the sample together
 constexpr uint32_t kCopyChunk = 32768;          // keys of one record of a range of equal keys
 constexpr uint32_t kSmallOver = 10;             // samples a range of a small sort (its ranges have room for three times their mean)
 
 template <class B>
 struct Sizes {
-  static constexpr uint32_t kLocal = sizeof(B) == 8 ? LS_LT64 : LS_LT32;  // keys one CTA sorts on chip
-  static constexpr uint32_t kSortThreads = sizeof(B) == 8 ? LS_NT64 : LS_NT32, kSortCtas = sizeof(B) == 8 ? LS_MINB64 : LS_MINB32;
-  static constexpr uint32_t kTarget = kLocal / 16 * 7;      // mean keys of a range
-  static constexpr int kTileRows = SP_KPT32 * 4 / (int)sizeof(B);
+  // Keys one CTA sorts on chip, and its CTAs: 256 threads, three on an SM. 2^28 u32 takes 3.37 ms so; with 512 threads and two CTAs
+  // 3.54, with four CTAs (fewer registers) 3.42, with two 3.48.
+  static constexpr uint32_t kLocal = sizeof(B) == 8 ? 4096 : 8192;
+  static constexpr uint32_t kSortThreads = 256, kSortCtas = 3;
+  static constexpr uint32_t kTarget = kLocal / 16 * 7;  // mean keys of a range (6/16: 2^28 u32 3.45 ms)
+  static constexpr int kTileRows = 64 / (int)sizeof(B);  // keys a thread of a tile
   static constexpr uint32_t kTile = kThreads * kTileRows;
   static constexpr int kLocalRows = (int)(kLocal / kSortThreads);
   static constexpr int kBlock = sizeof(B) == 8 ? 8 : 16;     // keys of one network of the on-chip sort
@@ -405,6 +384,9 @@ struct MapSmem {
 };
 constexpr uint32_t kNone = 0xffffu, kWhole = 0xfffeu;  // no part; nor will there be one (the keys are equal)
 
+// Latency: a chain of small steps by one CTA, 22 to 32 us at the first level of a large sort (its sample is read from HBM) and a few
+// without one. Maps that divide cells take 40 us and more; a warp a part and four samples at a time took 100003 zipf words from 78 to
+// 44 us.
 // Makes the map of src[0, len) for about k ranges: sm.tab and sm.part are its tables, `bins` its ranges (at most bin_room(k));
 // equal(bin, value) is called for each range that holds only keys equal to value. `salt` varies the sample. Every CTA that
 // calls it with the same arguments makes the same map; the CL CTAs of a cluster read a part of the sample each and hand it round.
@@ -799,7 +781,7 @@ __global__ void __launch_bounds__(kThreads) split_map(const BOf<T>* src, Tables 
     }
     KeyMap<T> map;
     uint32_t bins;
-    make_map<T>(sm, src + __ldcg(&rec->start), __ldcg(&rec->len), k, s, SP_OVER, max_sample, map, bins, [&](uint32_t b, B x) {
+    make_map<T>(sm, src + __ldcg(&rec->start), __ldcg(&rec->len), k, s, kOver, max_sample, map, bins, [&](uint32_t b, B x) {
       v.eq[bin0 + b] = 1u;
       v.value[bin0 + b] = x;
     });
@@ -833,6 +815,8 @@ __device__ __forceinline__ uint32_t find_segment(const SegRec* seg, uint32_t nse
   return lo;
 }
 
+// Every key's range, counted: reads the keys once. Bound by shared memory (a cell and a count each, seven wavefronts a row of 32)
+// 62 to 70 % of the rate, half the copy bandwidth: 2^25 u32 in 35 to 40 us. Three CTAs on an SM hide its loads, eight under way a thread.
 template <class T>
 __global__ void __launch_bounds__(kThreads, 3) split_count(const BOf<T>* src, Tables t, Level v, const Queue* q) {
   using B = BOf<T>;
@@ -971,10 +955,14 @@ struct TileSmem {
 };
 
 // One tile: `here` keys in registers (row j, thread tid: key j * kThreads + tid). Counts them by range with one shared atomic
-// each (its old value is the key's place in the tile's part of the range), reserves every range's share with reserve(range,
+// each, reserves every range's share with reserve(range,
 // count), groups the keys by range in shared memory, calls between(), then puts each key with put(range, first, key, index):
 // the tile's part of the range is key indexes [.., ..) of the groups and starts at `first` - index of its first.
 // The reservation's round trip to L2 is hidden behind the grouping, the next tile's loads (between) behind the writes.
+// Bound by shared-memory wavefronts: of random cells and counters, a row of 32 keys takes about 3.5 for the cell, 2.5 for the
+// count, 2.8 for the place, 3.5 for the write and 2 to 4 for reading back in order: 17 in all, 69 % of the rate at 2^25 u32 (96 us). A place from a second atomic (2.8)
+// costs less than the counter's start read again (3.5), and leaves half the registers for what is remembered of each key: 2^28 u32
+// 3.37 to 3.10 ms, 2^27 f32 1.87 to 1.72.
 template <class T, bool VALUE, bool PARTS_, bool COUNT_EQUAL, class E, class Reserve, class Between, class Put>
 __device__ __forceinline__ void scatter_tile(TileSmem<BOf<T>>& sm, const KeyMap<T>& map, const E* tab, const Part<BOf<T>>* part,
                                              uint32_t bins, const BOf<T> (&key)[Sizes<BOf<T>>::kTileRows], uint32_t here,
@@ -1109,7 +1097,7 @@ struct ScatterSmem {
 };
 
 template <class T>
-__global__ void __launch_bounds__(kThreads, SP_MINB) split_scatter(const BOf<T>* src, BOf<T>* dst, Tables t, Level v, Queue* q) {
+__global__ void __launch_bounds__(kThreads, kTileCtas) split_scatter(const BOf<T>* src, BOf<T>* dst, Tables t, Level v, Queue* q) {
   using B = BOf<T>;
   constexpr int ROWS = Sizes<B>::kTileRows;
   extern __shared__ __align__(16) unsigned char split_dyn[];
@@ -1202,7 +1190,7 @@ union SmallSmem {
 };
 
 template <class T, uint32_t CL>
-__global__ void __cluster_dims__(CL) __launch_bounds__(kThreads, SP_MINB) split_small(const BOf<T>* src, BOf<T>* area, uint32_t n, uint32_t k, Small* st, uint32_t tile_keys,
+__global__ void __cluster_dims__(CL) __launch_bounds__(kThreads, kTileCtas) split_small(const BOf<T>* src, BOf<T>* area, uint32_t n, uint32_t k, Small* st, uint32_t tile_keys,
                                                                  Queue* q) {
   using B = BOf<T>;
   constexpr int ROWS = Sizes<B>::kTileRows;
@@ -1433,6 +1421,10 @@ struct BinMap {
   }
 };
 
+// Bound by shared-memory wavefronts and issue slots together (21 wavefronts and 84 instructions a row of 32 keys, 59 % and 56 % of their rates at 2^25 u32): count 2.5,
+// place 2.8 and write 3.5 of them, networks 4, counters 2. Two counters share a word, eight are scanned with one 16-byte access, and
+// blocks are permuted, not padded: 30 to 21 wavefronts, 101 to 84 instructions, 2^28 u32 3.62 to 3.37 ms, 2^20 43.6 to 35.3 us.
+// 64-bit keys use networks of eight and two bins a key (a comparison is six instructions): 2^26 f64 2.00 to 1.87 ms.
 // Sorts `len` keys (row j, thread tid: key j * NT + tid, as the map orders them) into dst[off, off + len). Calls between() once
 // the keys have left their registers. Every bin holds about one key, so after one counting pass each key is close to its place, and
 // networks over neighbouring blocks finish the order without knowing the bins.
@@ -1802,6 +1794,8 @@ __device__ __forceinline__ void leave_small(Small* st, uint32_t bins, uint32_t t
   }
 }
 
+// Latency: a chain of reads (ranges, counts) and one range's sort a CTA, 9 us of the 29 at 2^20 keys. Each CTA reads what it needs of
+// all ranges in one round, its turn's answer is not waited for, and long ranges of equal keys are shared by all CTAs.
 // The ranges of a small sort: their starts are the scan of their counts, which every CTA makes for itself.
 template <class T>
 __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<BOf<T>>::kSortCtas) local_small(BOf<T>* d, const BOf<T>* area, uint32_t n, Small* st, Queue* q) {
@@ -2003,9 +1997,10 @@ cudaError_t launch_t(const SplitArgs& a, SplitResult* out) {
     Small* st = reinterpret_cast<Small*>(base + lay.small_at);
     B* area = reinterpret_cast<B*>(base + lay.area_at);
     const uint32_t n = (uint32_t)a.n, tiles = (n + tile_keys - 1u) / tile_keys, k = small_count<B>(a.n, a.sms);
-    // CTAs that read the sample each keep L2 busy once every SM has two of them; a cluster's CTAs share SMs where others are idle
+    // Once every SM has two CTAs that read the whole sample, L2 is busy with it: a cluster reads it once (2^20 u32 33.0 to 29.3 us,
+    // 2^21 44.7 to 39.3). With fewer CTAs a cluster's share SMs while others stay idle (300007 f64 28.4 to 33.3 us).
     if (tiles > sms) {
-      const uint32_t ctas = (least(sms * SP_MINB, tiles) + kCluster - 1u) / kCluster * kCluster;
+      const uint32_t ctas = (least(sms * kTileCtas, tiles) + kCluster - 1u) / kCluster * kCluster;
       go(split_small<T, kCluster>, ctas, kThreads, sizeof(SmallSmem<B>), (const B*)d, area, n, k, st, tile_keys, a.q);
     } else {
       go(split_small<T, 1>, tiles, kThreads, sizeof(SmallSmem<B>), (const B*)d, area, n, k, st, tile_keys, a.q);
@@ -2018,6 +2013,8 @@ cudaError_t launch_t(const SplitArgs& a, SplitResult* out) {
     out->from_dn = 0u;
     return e;
   }
+  // One level reaches ranges that fit on chip up to kMaxBins of them. A plain sort past 2^21 keys takes two levels even so: fewer,
+  // larger ranges a level write longer runs.
   const uint32_t levels = a.n > (size_t)kMaxBins * Sizes<B>::kTarget || (plain && a.n > (1u << 21)) ? 2u : a.n > Sizes<B>::kLocal ? 1u : 0u;
   while (tile_keys > 4u * kThreads && a.n / tile_keys < 2u * sms) tile_keys -= 2u * kThreads;
   const Tables t = lay.tables(a.scratch, tile_keys);
@@ -2042,7 +2039,7 @@ cudaError_t launch_t(const SplitArgs& a, SplitResult* out) {
     go(split_map<T>, gs, kThreads, sizeof(MapSmem<B>) + sample * sizeof(B), src, t, lv[l], plain && !l ? (uint32_t)a.n : 0u, levels, sample, a.q);
     go(split_count<T>, least(sms * 3u, tiles), kThreads, 0, src, t, lv[l], (const Queue*)a.q);
     go(split_starts<T>, gs, kThreads, 0, t, lv[l], lv[1], levels, a.q);
-    go(split_scatter<T>, least(sms * SP_MINB, tiles), kThreads, sizeof(ScatterSmem<B>), src, dst, t, lv[l], a.q);
+    go(split_scatter<T>, least(sms * kTileCtas, tiles), kThreads, sizeof(ScatterSmem<B>), src, dst, t, lv[l], a.q);
   }
   const bool one = plain && !levels;
   go(local_sort<T>, one ? 1u : least(sms * Sizes<B>::kSortCtas, lay.buckets), Sizes<B>::kSortThreads, sizeof(LocalSmem<B>), d, dn, a.bound, t, one ? (uint32_t)a.n : 0u, a.q);
