@@ -52,7 +52,7 @@ typedef struct gqs_config {
   int32_t variant;     /* -1: per sort, the tuned variant for its key type and size; else fixed */
   uint32_t timeout_ms; /* device-side no-progress limit for bounded waits; 0 means 4000 */
   uint32_t sync;       /* 1 (default): *_dev calls wait for the stream and return the device status */
-  uint32_t timing;     /* 1: time the persistent kernel with CUDA events (gqs_stats.kernel_ms) */
+  uint32_t timing;     /* 1: time the sort's kernels with CUDA events (gqs_stats.kernel_ms) */
   uint32_t reserved[4];
 } gqs_config;
 
@@ -66,7 +66,7 @@ typedef struct gqs_stats {
   uint64_t algo_bytes; /* key bytes * 2 * (part_keys + local_keys + tiny_keys) */
   uint32_t part_jobs, local_jobs, fill_chunks, max_depth;
   uint32_t status, variant, grid, threads;
-  double kernel_ms; /* persistent-kernel time from CUDA events, or -1 when timing is off */
+  double kernel_ms; /* the sort's kernels' time from CUDA events, or -1 when timing is off */
 } gqs_stats;
 
 typedef struct gqs_variant_desc {
@@ -107,7 +107,7 @@ gqs_status gqs_sort_f32_dev(gqs_ctx* ctx, float* d, float* scratch, size_t n, vo
 gqs_status gqs_sort_f64_dev(gqs_ctx* ctx, double* d, double* scratch, size_t n, void* stream);
 
 /* Segmented sorts: keys[offsets[i], offsets[i+1]) is sorted independently for each of the
- * nseg segments, all in one persistent launch. offsets holds nseg + 1 non-decreasing entries
+ * nseg segments, all in one chain of launches. offsets holds nseg + 1 non-decreasing entries
  * (device memory for *_dev, host memory otherwise) with offsets[nseg] <= n, where n is the
  * length of keys (and of scratch). No reference counterpart: the reference sorts one array per
  * call; this is the batched form of the same GPUQSort<T> path. */
@@ -126,7 +126,7 @@ gqs_status gqs_sort_segments_f64(gqs_ctx* ctx, double* keys, size_t n, const uin
  * so values 0..n-1 give a stable argsort (the sorting permutation). Host-pointer forms sort both
  * host arrays in place; *_dev forms take device arrays and a stream (cfg.sync as above). Each
  * pair is packed into one 64-bit word (the key's order-preserving map above the value) and
- * the words are sorted by the same persistent kernel. No reference counterpart: the reference
+ * the words are sorted as 64-bit keys. No reference counterpart: the reference
  * sorts keys only; this is the key-value variant of its GPUQSort<T> path. */
 gqs_status gqs_sort_pairs_u32(gqs_ctx* ctx, uint32_t* keys, uint32_t* values, size_t n);
 gqs_status gqs_sort_pairs_f32(gqs_ctx* ctx, float* keys, uint32_t* values, size_t n);
@@ -156,10 +156,10 @@ gqs_status gqs_sort_u32_noalloc(uint32_t* d, size_t n, void* stream);
 
 /* ---- Batched sort, captured once as a CUDA graph ------------------------------------------
  * A batch sorts up to max_segments independent arrays (segments) of one key type, holding up to
- * max_keys keys in total, in one persistent launch. It owns its device memory: a key arena of
+ * max_keys keys in total, in one chain of launches. It owns its device memory: a key arena of
  * max_keys keys that the caller fills (gqs_batch_keys), its scratch, the job records, ticket
  * ring and status block. The work of one batch (copy of the segment table from pinned host
- * memory, clearing of the status block and ring, the seed kernel, the persistent kernel, the
+ * memory, clearing of the status block and ring, the split, the seed and persistent kernels, the
  * read-back of the status block) is captured once per kernel variant as a CUDA graph;
  * gqs_batch_launch replays it with a single cudaGraphLaunch. The segment table is data, so
  * batches of any shape up to the maxima replay the same graph.
@@ -317,7 +317,7 @@ typedef struct gqs_level {
   uint32_t reserved;
   uint64_t local_keys; /* the keys they sorted */
   double first_ms;     /* a first and the last job completion at this depth, ms after the */
-  double last_ms;      /* persistent kernel started */
+  double last_ms;      /* kernels started */
 } gqs_level;
 
 /* Per-level statistics of the context's last sort, the counterpart of the reference's optional
