@@ -8,7 +8,7 @@ uniformly over [0, 2^32) from a fixed seed. A step is one sort of that array.
             timed interval; 1 GiB of keys exceeds the 129 MB L2, and the restore copy rewrites it)
   e2e       the same metric through the host-pointer C ABI call (pinned host buffer -> HBM,
             sort, -> host), wall clock per call
-  roofline  algorithmic bytes of the persistent kernel (key bytes * 2 * keys read by partition
+  roofline  algorithmic bytes of the sort's kernels (key bytes * 2 * keys read by partition
             chunks + keys sorted on chip + keys sorted in registers, from the kernel's own
             counters) / its CUDA-event duration, against the measured HBM copy bandwidth
 
@@ -111,7 +111,7 @@ def measured_peak():
 
 
 def ncu_traffic(workload_key):
-    """Per-launch DRAM bytes of the persistent kernel from a committed ncu summary, if any."""
+    """DRAM bytes of one sort from a committed ncu summary, if any."""
     path = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     try:
         with open(path) as f:
@@ -619,9 +619,9 @@ def run_pairs(args, gqs_ctypes, rank, local, world, dist, barrier):
             "config": {"workload": f"key-value sort of 2^{args.log2n} pairs", "keys": n,
                        "l2": "inputs larger than L2 (rewritten from pristine copies before every step)"},
             "roofline": {"bound": "hbm", "achieved": ab / (km / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
-                         "frac": ab / (km / 1e3) / 1e9 / peak, "kernel": "gqs::persistent_kernel (u64 words)",
+                         "frac": ab / (km / 1e3) / 1e9 / peak, "kernel": "gqs split of u64 words",
                          "kernel_ms": km, "algo_bytes_per_launch": ab, "peak_source": peak_src},
-            "check": check, "gpu_launches": 4 * args.steps}
+            "check": check, "gpu_launches": (2 + split_kernels(n, 8)) * args.steps}  # with pack and unpack
 
 
 def run_batched(args, gqs_ctypes, rank, local, world, dist, barrier, clocks=None, steps=None, warmup=None):
@@ -762,7 +762,7 @@ def run_batched(args, gqs_ctypes, rank, local, world, dist, barrier, clocks=None
                    "graph": "one cudaGraphLaunch per step", "parallelism": f"replicas x{world}"},
         "autotune": tune,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": ncu_traffic("batched_u32"), "kernel": "gqs::persistent_kernel (graph replay)",
+                     "traffic": ncu_traffic("batched_u32"), "kernel": "gqs split (graph replay)",
                      "kernel_ms": km, "algo_bytes_per_launch": ab, "peak_source": peak_src},
         "kernel_ms": km,
         "plain_per_array": {"gkeys_s": n / (plain_ms / 1e3) / 1e9, "ms": plain_ms, "calls": nseg,
@@ -948,12 +948,21 @@ class PlainRunner:
                        if flush is None else "L2 flushed before every step (256 MiB write)")}
 
 
+def split_kernels(n, esize):
+    """Kernels of one plain sort of n keys (csrc/gqs_split.cu; the persistent kernel that may follow is not counted)."""
+    if n <= (8192 if esize == 4 else 4096):
+        return 1
+    if n <= (1 << 21 if esize == 4 else 1 << 19):
+        return 2
+    return 5 if esize == 8 and n <= 1024 * 1792 else 9
+
+
 def roofline_of(r, peak, peak_src, traffic=None):
     km = float(np.mean(r["kernel_ms"]))
     ab = float(np.mean(r["algo_bytes"]))
     achieved = ab / (km / 1e3) / 1e9
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": traffic, "kernel": "gqs::persistent_kernel", "kernel_ms": km, "algo_bytes_per_launch": ab,
+            "traffic": traffic, "kernel": "gqs split: map, count, starts, scatter (two levels), local_sort", "kernel_ms": km, "algo_bytes_per_launch": ab,
             "peak_source": peak_src,
             "per_unit": f"{r['esize']} B x 2 per key per pass (partition chunks + on-chip sort + register sort)"}
 
@@ -1140,7 +1149,7 @@ def main():
         "roofline": roofline,
         "cpu_baseline": cpu,
         "e2e": e2e,
-        "gpu_launches": 2 * args.steps,
+        "gpu_launches": split_kernels(n, r["esize"]) * args.steps,
         "clocks": clk,
         "check": r["check"],
         "stats": {k: stats_last[k] for k in ("part_keys", "local_keys", "tiny_keys", "fill_keys", "chunks",
