@@ -146,6 +146,7 @@ struct gqs_ctx {
 #endif
   void* split_buf = nullptr;  // scratch of the top split of small sorts (gqs_split.cu)
   size_t split_bytes = 0;
+  bool split_uncleared = false;  // its counters have not been zeroed since it was allocated
   bool top_split = true;
   int variant[4] = {0, 0, 0, 0};  // per key type, and the internal packed pairs
   bool auto_variant[4] = {true, true, true, true};  // pick per call from the tuning table
@@ -178,14 +179,13 @@ cudaError_t launch_quicksort(gqs_ctx* c, int dtype, const gqs::LaunchParams& p, 
   return e == cudaSuccess ? gqs::launch_sort(dtype, p) : e;
 }
 
-// Grows the split's scratch; no sort is using it.
+// Grows the split's scratch; no sort is using it. New scratch is cleared on the stream of the
+// first sort that uses it: nothing else orders that sort behind the clearing (the default stream
+// does not wait for a non-blocking one, nor the other way round).
 gqs_status grow_split(gqs_ctx* c, size_t bytes) {
-  const void* const old = c->split_buf;
-  const size_t had = c->split_bytes;
-  gqs_status st = grow(&c->split_buf, &c->split_bytes, bytes);
-  if (st == GQS_OK && (c->split_buf != old || c->split_bytes != had))
-    st = cuda_status(cudaMemset(c->split_buf, 0, gqs::split_clear_bytes()));
-  return st;
+  if (c->split_buf && c->split_bytes >= bytes) return GQS_OK;
+  c->split_uncleared = true;
+  return grow(&c->split_buf, &c->split_bytes, bytes);
 }
 
 gqs_status wait_pending_locked(gqs_ctx* c) {
@@ -332,6 +332,11 @@ gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, co
     sa.sms = c->num_sms;
     sa.stream = stream;
     gqs::SplitResult left{};
+    if (c->split_uncleared) {
+      e = cudaMemsetAsync(c->split_buf, 0, gqs::split_clear_bytes(), stream);
+      if (e != cudaSuccess) return cuda_status(e);
+      c->split_uncleared = false;
+    }
     if ((e = gqs::split_launch(dtype, sa, &left)) != cudaSuccess) return cuda_status(e);
     p.offsets = left.table;
     p.nseg_dev = left.count;
@@ -764,6 +769,12 @@ gqs_status gqs_reserve(gqs_ctx* c, int dtype, size_t n, size_t nseg, int with_bu
     if (nseg_in > 1) bytes = std::max(bytes, gqs::split_scratch_bytes(dtype, m, nseg_in, false, c->num_sms));
     gqs_status st = grow_split(c, bytes);
     if (st != GQS_OK) return st;
+    if (c->split_uncleared) {  // here, so that a sort that follows, or is captured, has it behind it
+      cudaError_t e = cudaMemsetAsync(c->split_buf, 0, gqs::split_clear_bytes(), c->stream);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+      if (e != cudaSuccess) return cuda_status(e);
+      c->split_uncleared = false;
+    }
     nseg = std::max(nseg_in, m / 4096 + 1);
   }
   const size_t cap = job_capacity(vi, n, nseg ? nseg : 1);

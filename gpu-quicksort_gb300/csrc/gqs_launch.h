@@ -126,7 +126,9 @@ struct SplitResult {
   uint32_t from_dn;                 // 1: their keys are in dn
 };
 size_t split_scratch_bytes(int dtype, size_t n, size_t nseg, bool plain, int sms);
-size_t split_clear_bytes();  // the scratch's first bytes, to be zeroed once when it is allocated
+// The scratch's first bytes, to be zeroed before the first sort that uses it, in that sort's stream
+// or one that it follows.
+size_t split_clear_bytes();
 cudaError_t split_launch(int dtype, const SplitArgs& a, SplitResult* out);
 constexpr size_t kDtypeBytes(int dtype) { return dtype == DT_U32 || dtype == DT_F32 ? 4 : 8; }
 

@@ -1841,6 +1841,11 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
     return;
   }
   uint32_t at = block_scan<NT>(sum, sm.wsum, total);
+  if (total != n) {  // the counters were not zero when the sort began: no start below can be relied on
+    if (blockIdx.x == 0 && tid == 0) set_error(q, ST_INTERNAL, total);
+    leave_small(st, bins, turn);
+    return;
+  }
 #pragma unroll
   for (uint32_t i = 0; i < R; ++i) {
     const uint32_t b = tid * per + i;
