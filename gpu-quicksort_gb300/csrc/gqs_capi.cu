@@ -14,6 +14,7 @@
 #include <new>
 
 #include "gqs.h"
+#include "gqs_counters.h"
 #include "gqs_device.cuh"
 #include "gqs_host.h"
 #include "gqs_launch.h"
@@ -146,7 +147,7 @@ struct gqs_ctx {
 #endif
   void* split_buf = nullptr;  // scratch of the top split of small sorts (gqs_split.cu)
   size_t split_bytes = 0;
-  bool split_uncleared = false;  // its counters have not been zeroed since it was allocated
+  gqs::SplitCounters split_counters;  // those at its head
   bool top_split = true;
   int variant[4] = {0, 0, 0, 0};  // per key type, and the internal packed pairs
   bool auto_variant[4] = {true, true, true, true};  // pick per call from the tuning table
@@ -184,8 +185,16 @@ cudaError_t launch_quicksort(gqs_ctx* c, int dtype, const gqs::LaunchParams& p, 
 // does not wait for a non-blocking one, nor the other way round).
 gqs_status grow_split(gqs_ctx* c, size_t bytes) {
   if (c->split_buf && c->split_bytes >= bytes) return GQS_OK;
-  c->split_uncleared = true;
+  c->split_counters.spoil();
   return grow(&c->split_buf, &c->split_bytes, bytes);
+}
+
+// Whether work enqueued on `stream` is captured into a graph instead of run.
+bool capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+  (void)cudaGetLastError();
+  return true;
 }
 
 gqs_status wait_pending_locked(gqs_ctx* c) {
@@ -210,6 +219,7 @@ gqs_status wait_pending_locked(gqs_ctx* c) {
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, c->ev_begin, c->ev_end) == cudaSuccess) s.kernel_ms = ms;
   }
+  if (s.status != GQS_OK) c->split_counters.spoil();
   c->last = s;
   for (int i = 0; i < 32; ++i) c->last_prof[i] = c->q_host->prof[i];
   for (int i = 0; i < 4; ++i) c->last_phase[i] = c->q_host->phase[i];
@@ -332,12 +342,17 @@ gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, co
     sa.sms = c->num_sms;
     sa.stream = stream;
     gqs::SplitResult left{};
-    if (c->split_uncleared) {
-      e = cudaMemsetAsync(c->split_buf, 0, gqs::split_clear_bytes(), stream);
-      if (e != cudaSuccess) return cuda_status(e);
-      c->split_uncleared = false;
+    const bool captured = capturing(stream);
+    e = c->split_counters.enqueue<cudaError_t>(
+        captured, [&] { return cudaMemsetAsync(c->split_buf, 0, gqs::split_clear_bytes(), stream); },
+        [&] { return gqs::split_launch(dtype, sa, &left); });
+    if (e != cudaSuccess) {
+      const gqs_status failed = cuda_status(e);
+      // the next sort, on whatever stream, finds none of this one's kernels still running
+      if (!captured) cudaStreamSynchronize(stream);
+      (void)cudaGetLastError();
+      return failed;
     }
-    if ((e = gqs::split_launch(dtype, sa, &left)) != cudaSuccess) return cuda_status(e);
     p.offsets = left.table;
     p.nseg_dev = left.count;
     p.nseg = left.most;
@@ -769,11 +784,11 @@ gqs_status gqs_reserve(gqs_ctx* c, int dtype, size_t n, size_t nseg, int with_bu
     if (nseg_in > 1) bytes = std::max(bytes, gqs::split_scratch_bytes(dtype, m, nseg_in, false, c->num_sms));
     gqs_status st = grow_split(c, bytes);
     if (st != GQS_OK) return st;
-    if (c->split_uncleared) {  // here, so that a sort that follows, or is captured, has it behind it
+    if (c->split_counters.unclear()) {  // here, so that a sort that follows, or is captured, has it behind it
       cudaError_t e = cudaMemsetAsync(c->split_buf, 0, gqs::split_clear_bytes(), c->stream);
       if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
       if (e != cudaSuccess) return cuda_status(e);
-      c->split_uncleared = false;
+      c->split_counters.cleared();
     }
     nseg = std::max(nseg_in, m / 4096 + 1);
   }

@@ -1,0 +1,31 @@
+// Whether the counters at the head of the split's scratch are zero, which a small sort relies on and leaves behind it when it runs to
+// its end. They are not in new scratch, nor after a sort that was enqueued only in part or failed. Host logic only.
+#pragma once
+
+namespace gqs {
+
+class SplitCounters {
+  bool unclear_ = false;
+
+ public:
+  void spoil() { unclear_ = true; }
+  bool unclear() const { return unclear_; }
+  void cleared() { unclear_ = false; }
+
+  // Enqueues one sort with launch(), behind clear() if the counters may not be zero; both return a status, S{} for success. In a
+  // stream that is being captured (`captured`) neither has run when this returns: the graph clears them for itself.
+  template <class S, class Clear, class Launch>
+  S enqueue(bool captured, Clear&& clear, Launch&& launch) {
+    const bool was = unclear_;
+    if (was) {
+      const S e = clear();
+      if (e != S{}) return e;
+    }
+    unclear_ = true;
+    const S e = launch();
+    if (e == S{}) unclear_ = was && captured;
+    return e;
+  }
+};
+
+}  // namespace gqs
