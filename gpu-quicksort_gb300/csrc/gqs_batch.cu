@@ -130,6 +130,10 @@ gqs_status GraphSort::capture(int dtype, int variant) {
   const int bps = blocks_per_sm(dtype, variant);
   if (!bps) return GQS_ERR_NO_DEVICE;
   if (!keys_ || !scratch_) return GQS_ERR_INVALID;
+  if (split_) {
+    const cudaError_t prepared = split_prepare(dtype);
+    if (prepared != cudaSuccess) return cuda_status(prepared);
+  }
   LaunchParams p{};
   p.d = keys_;
   p.dn = scratch_;

@@ -148,6 +148,7 @@ struct gqs_ctx {
   void* split_buf = nullptr;  // scratch of the top split of small sorts (gqs_split.cu)
   size_t split_bytes = 0;
   gqs::SplitCounters split_counters;  // those at its head
+  bool split_prepared[4] = {};        // per key type: its kernels may be launched on this device
   bool top_split = true;
   int variant[4] = {0, 0, 0, 0};  // per key type, and the internal packed pairs
   bool auto_variant[4] = {true, true, true, true};  // pick per call from the tuning table
@@ -269,6 +270,11 @@ gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, co
   if (!c->blocks_per_sm[dtype][v]) {
     c->blocks_per_sm[dtype][v] = gqs::variant_prepare(dtype, v);
     if (!c->blocks_per_sm[dtype][v]) return GQS_ERR_NO_DEVICE;
+  }
+  if (split && !c->split_prepared[dtype]) {
+    const cudaError_t e = gqs::split_prepare(dtype);
+    if (e != cudaSuccess) return cuda_status(e);
+    c->split_prepared[dtype] = true;
   }
   gqs_status st = GQS_OK;
   const bool need_jobs = c->job_cap < cap;
@@ -789,6 +795,11 @@ gqs_status gqs_reserve(gqs_ctx* c, int dtype, size_t n, size_t nseg, int with_bu
       if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
       if (e != cudaSuccess) return cuda_status(e);
       c->split_counters.cleared();
+    }
+    if (!c->split_prepared[dtype]) {
+      const cudaError_t e = gqs::split_prepare(dtype);
+      if (e != cudaSuccess) return cuda_status(e);
+      c->split_prepared[dtype] = true;
     }
     nseg = std::max(nseg_in, m / 4096 + 1);
   }

@@ -129,6 +129,9 @@ size_t split_scratch_bytes(int dtype, size_t n, size_t nseg, bool plain, int sms
 // The scratch's first bytes, to be zeroed before the first sort that uses it, in that sort's stream
 // or one that it follows.
 size_t split_clear_bytes();
+// Raises the shared-memory limits of the split's kernels on the current device, to which they belong: each owner of a scratch
+// calls it before its first split_launch.
+cudaError_t split_prepare(int dtype);
 cudaError_t split_launch(int dtype, const SplitArgs& a, SplitResult* out);
 constexpr size_t kDtypeBytes(int dtype) { return dtype == DT_U32 || dtype == DT_F32 ? 4 : 8; }
 

@@ -1968,18 +1968,20 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
 }
 
 template <class T>
+cudaError_t prepare_t() {
+  using B = BOf<T>;
+  cudaError_t e = allow_smem(split_scatter<T>, sizeof(ScatterSmem<B>));
+  if (e == cudaSuccess) e = allow_smem(split_map<T>, sizeof(MapSmem<B>) + Sizes<B>::kMaxSample * sizeof(B));
+  if (e == cudaSuccess) e = allow_smem(split_small<T, 1>, sizeof(SmallSmem<B>));
+  if (e == cudaSuccess) e = allow_smem(split_small<T, kCluster>, sizeof(SmallSmem<B>));
+  if (e == cudaSuccess) e = allow_smem(local_sort<T>, sizeof(LocalSmem<B>));
+  if (e == cudaSuccess) e = allow_smem(local_small<T>, sizeof(SmallSortSmem<B>));
+  return e;
+}
+
+template <class T>
 cudaError_t launch_t(const SplitArgs& a, SplitResult* out) {
   using B = BOf<T>;
-  static const cudaError_t attr = [] {
-    cudaError_t e = allow_smem(split_scatter<T>, sizeof(ScatterSmem<B>));
-    if (e == cudaSuccess) e = allow_smem(split_map<T>, sizeof(MapSmem<B>) + Sizes<B>::kMaxSample * sizeof(B));
-    if (e == cudaSuccess) e = allow_smem(split_small<T, 1>, sizeof(SmallSmem<B>));
-    if (e == cudaSuccess) e = allow_smem(split_small<T, kCluster>, sizeof(SmallSmem<B>));
-    if (e == cudaSuccess) e = allow_smem(local_sort<T>, sizeof(LocalSmem<B>));
-    if (e == cudaSuccess) e = allow_smem(local_small<T>, sizeof(SmallSortSmem<B>));
-    return e;
-  }();
-  if (attr != cudaSuccess) return attr;
   const bool plain = a.offsets == nullptr;
   const Layout<B> lay(a.n, a.nseg, plain, a.sms);
   char* const base = static_cast<char*>(a.scratch);
@@ -2068,6 +2070,15 @@ size_t split_scratch_bytes(int dtype, size_t n, size_t nseg, bool plain, int sms
 }
 
 size_t split_clear_bytes() { return sizeof(Small); }
+
+cudaError_t split_prepare(int dtype) {
+  switch (dtype) {
+    case DT_U32: return prepare_t<uint32_t>();
+    case DT_F32: return prepare_t<float>();
+    case DT_F64: return prepare_t<double>();
+    default: return prepare_t<uint64_t>();
+  }
+}
 
 cudaError_t split_launch(int dtype, const SplitArgs& a, SplitResult* out) {
   switch (dtype) {
