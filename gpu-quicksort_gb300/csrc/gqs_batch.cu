@@ -25,9 +25,8 @@ namespace gqs {
 GraphSort::~GraphSort() {
   if (ev_end_) cudaEventSynchronize(ev_end_);
   drop_graphs();
-  if (jobs_) cudaFree(jobs_);
+  if (records_) cudaFree(records_);
   if (ring_) cudaFree(ring_);
-  if (split_) cudaFree(split_);
   if (q_) cudaFree(q_);
   if (hdr_dev_) cudaFree(hdr_dev_);
   if (q_host_) cudaFreeHost(q_host_);
@@ -58,25 +57,33 @@ gqs_status GraphSort::init(int device, int num_sms, size_t max_keys, size_t max_
   pairs_ = pairs;
   timeout_ms_ = timeout_ms ? timeout_ms : 4000;
   table_words_ = 1 + (pairs ? 2 * max_segs : max_segs + 1);
-  // Job records and ring entries for the most demanding variant of any key type.
-  size_t cap = 0, ring = 0, split = 0;
+  // Job records and ring entries for the most demanding variant of any key type. They hold what the split leaves too: ranges of more
+  // than 4096 keys, each at most one root, where the records are made for jobs of a few hundred keys and the ring for their chunks.
+  size_t cap = 0, ring = 0, split = 0, keep = 0;
   const bool use_split = max_keys < (1ull << 31);
-  const size_t roots = use_split ? std::max(max_segs, max_keys / 4096 + 1) : max_segs;  // the split may leave so many ranges
-  for (int t = 0; t < 3 && use_split; ++t) split = std::max(split, split_scratch_bytes(t, max_keys, max_segs, false, num_sms));
-  for (int t = 0; t < 3; ++t)
+  for (int t = 0; t < 3; ++t) {
+    if (use_split) {
+      split = std::max(split, split_scratch_bytes(t, max_keys, max_segs, false, num_sms));
+      keep = std::max(keep, split_keep_bytes(t, max_keys, max_segs, num_sms));
+    }
     for (int v = 0; v < variant_count(t); ++v) {
       const VariantInfo vi = variant_info(t, v);
-      cap = std::max(cap, job_capacity(vi, max_keys, roots));
-      ring = std::max(ring, ticket_ring(vi, max_keys, roots));
+      cap = std::max(cap, job_capacity(vi, max_keys, max_segs));
+      ring = std::max(ring, ticket_ring(vi, max_keys, max_segs));
     }
+  }
   if (cap >= (1ull << 32) || ring > (1ull << 31)) return GQS_ERR_INVALID;
+  // One piece of memory for the split's tables and the job records, which are made when the split has finished: 168 MB instead of
+  // 312 at 2^27 keys. In front of the records, what the split leaves to them.
+  const size_t jobs = cap * sizeof(Job), rest = split > keep ? split - keep : 0;
+  record_bytes_ = std::max(jobs, rest) + ring * sizeof(unsigned long long);
   cudaError_t e;
-  if ((e = cudaMalloc(&jobs_, cap * sizeof(Job))) != cudaSuccess) return cuda_status(e);
+  if ((e = cudaMalloc(&records_, keep + std::max(jobs, rest))) != cudaSuccess) return cuda_status(e);
+  jobs_ = reinterpret_cast<Job*>(static_cast<char*>(records_) + keep);
   job_cap_ = cap;
   if ((e = cudaMalloc(&ring_, ring * sizeof(unsigned long long))) != cudaSuccess) return cuda_status(e);
   ring_len_ = ring;
-  if (split && (e = cudaMalloc(&split_, split)) != cudaSuccess) return cuda_status(e);
-  split_bytes_ = split;
+  split_ = use_split ? records_ : nullptr;
   if ((e = cudaMalloc(&q_, sizeof(Queue))) != cudaSuccess) return cuda_status(e);
   if ((e = cudaMalloc(&hdr_dev_, table_words_ * sizeof(unsigned long long))) != cudaSuccess) return cuda_status(e);
   if ((e = cudaMallocHost(&q_host_, sizeof(Queue))) != cudaSuccess) return cuda_status(e);

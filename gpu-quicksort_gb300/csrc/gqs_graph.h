@@ -41,8 +41,8 @@ class GraphSort {
   unsigned long long* table() const { return hdr_host_ + 1; }
   size_t max_segments() const { return max_segs_; }
   size_t max_keys() const { return max_keys_; }
-  // Device memory of the job records, the ticket ring and the split's scratch.
-  size_t record_bytes() const { return job_cap_ * sizeof(Job) + ring_len_ * sizeof(unsigned long long) + split_bytes_; }
+  // Device memory of the job records, which the split's tables share, and the ticket ring.
+  size_t record_bytes() const { return record_bytes_; }
 
   // Checks the table on the host: every segment inside the arena, at most max_keys keys.
   gqs_status validate(int dtype, size_t nseg, unsigned long long* keys_out) const;
@@ -70,12 +70,13 @@ class GraphSort {
   void* keys_ = nullptr;
   void* scratch_ = nullptr;
   size_t arena_bytes_ = 0;
+  void* records_ = nullptr;  // job records, and in the same place before them the split's tables
+  size_t record_bytes_ = 0;
   Job* jobs_ = nullptr;
   size_t job_cap_ = 0;
   unsigned long long* ring_ = nullptr;
   size_t ring_len_ = 0;
   void* split_ = nullptr;  // scratch of the split (null: too many keys for it)
-  size_t split_bytes_ = 0;
   Queue* q_ = nullptr;
   Queue* q_host_ = nullptr;
   unsigned long long* hdr_dev_ = nullptr;

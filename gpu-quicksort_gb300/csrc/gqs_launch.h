@@ -129,6 +129,9 @@ size_t split_scratch_bytes(int dtype, size_t n, size_t nseg, bool plain, int sms
 // The scratch's first bytes, to be zeroed before the first sort that uses it, in that sort's stream
 // or one that it follows.
 size_t split_clear_bytes();
+// Of the scratch of a segmented sort, the first bytes, which hold what the split leaves to the persistent kernel. The rest is
+// free once the split's last kernel has finished: the persistent kernel's own records may lie there.
+size_t split_keep_bytes(int dtype, size_t n, size_t nseg, int sms);
 // Raises the shared-memory limits of the split's kernels on the current device, to which they belong: each owner of a scratch
 // calls it before its first split_launch.
 cudaError_t split_prepare(int dtype);

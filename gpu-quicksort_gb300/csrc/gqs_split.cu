@@ -2071,6 +2071,10 @@ size_t split_scratch_bytes(int dtype, size_t n, size_t nseg, bool plain, int sms
 
 size_t split_clear_bytes() { return sizeof(Small); }
 
+size_t split_keep_bytes(int dtype, size_t n, size_t nseg, int sms) {
+  return kDtypeBytes(dtype) == 4 ? Layout<uint32_t>(n, nseg, false, sms).seg_at[0] : Layout<uint64_t>(n, nseg, false, sms).seg_at[0];
+}
+
 cudaError_t split_prepare(int dtype) {
   switch (dtype) {
     case DT_U32: return prepare_t<uint32_t>();
