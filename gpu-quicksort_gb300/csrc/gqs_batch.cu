@@ -189,6 +189,7 @@ gqs_status GraphSort::capture(int dtype, int variant) {
     p.nseg = left.most;
     p.pairs = 1;
     p.from_dn = left.from_dn;
+    p.after_kernel = 1;
   }
   if (first == cudaSuccess && (!split_ || p.nseg)) keep(launch_sort(dtype, p));
   keep(cudaMemcpyAsync(q_host_, q_, sizeof(Queue), cudaMemcpyDeviceToHost, cap_stream_));

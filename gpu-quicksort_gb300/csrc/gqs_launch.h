@@ -39,7 +39,8 @@ struct LaunchParams {
   uint32_t nseg;                      // segments (with nseg_dev: the most the launch may see)
   const unsigned long long* nseg_dev; // optional: segment count read on the device (replayable graphs)
   uint32_t pairs;                     // 1: offsets holds (start, end) per segment, 2 * nseg entries
-  uint32_t from_dn;                   // 1: the segments' keys are in dn (buckets of a top split)
+  uint32_t from_dn;                   // 1: the segments' keys are in dn (ranges of one counted level of the split)
+  uint32_t after_kernel;              // 1: the work in front of it in the stream is a kernel, so it may launch early
   int variant;
   int grid;
   cudaStream_t stream;

@@ -45,9 +45,9 @@ struct VariantOps {
     a.n = p.check_n ? p.check_n : p.n;
     const uint32_t nseg = p.offsets ? p.nseg : 1u;
     const uint32_t seed_blocks = (nseg + 7u) / 8u;  // 8 warps per 256-thread block, one per segment
-    // After a top split the seed kernel follows split_scatter as a programmatic dependent
-    // launch; the persistent kernel follows the seed kernel so whenever no event lies between.
-    cudaError_t e = launch_kernel(p.from_dn != 0, seed_kernel<C>, dim3(seed_blocks), dim3(256), 0, p.stream, a,
+    // Right behind the split's last kernel (in a batch's graph) the seed kernel is a programmatic dependent launch; a context
+    // clears its ring in between. The persistent kernel follows the seed kernel so whenever no event lies between.
+    cudaError_t e = launch_kernel(p.after_kernel != 0, seed_kernel<C>, dim3(seed_blocks), dim3(256), 0, p.stream, a,
                                   p.offsets, p.nseg_dev, nseg, (unsigned long long)p.n, p.pairs, p.from_dn);
     if (e != cudaSuccess) return e;
     if (p.ev_begin) cudaEventRecord(p.ev_begin, p.stream);
