@@ -149,7 +149,6 @@ struct gqs_ctx {
   size_t split_bytes = 0;
   gqs::SplitCounters split_counters;  // those at its head
   bool split_prepared[4] = {};        // per key type: its kernels may be launched on this device
-  bool top_split = true;
   int variant[4] = {0, 0, 0, 0};  // per key type, and the internal packed pairs
   bool auto_variant[4] = {true, true, true, true};  // pick per call from the tuning table
   int blocks_per_sm[4][kMaxVariants] = {};
@@ -244,10 +243,12 @@ gqs_status drain(gqs_ctx* c, gqs_status st) {
   return st;
 }
 
-// Which sorts start with the split. A context with a fixed kernel variant keeps to it above 2^21 keys and below 2^15.
+// Which sorts start with the split: below 2^31 keys, all but the plain sorts of a context with a fixed kernel variant above 2^21 keys
+// and below 2^15.
+constexpr size_t kSplitKeys = (1ull << 31) - 1, kFixedLeast = 1u << 15, kFixedMost = 1u << 21;
 bool use_split(const gqs_ctx* c, int dtype, size_t n, bool plain) {
-  if (!c->top_split || n >= (1ull << 31)) return false;
-  return !plain || c->auto_variant[dtype] || (n >= (1u << 15) && n <= (1u << 21));
+  if (n > kSplitKeys) return false;
+  return !plain || c->auto_variant[dtype] || (n >= kFixedLeast && n <= kFixedMost);
 }
 
 // Validates, grows pools, and enqueues one sort on `stream`. Caller holds the lock. `waits`: the
@@ -781,13 +782,13 @@ gqs_status gqs_reserve(gqs_ctx* c, int dtype, size_t n, size_t nseg, int with_bu
     if (!c->blocks_per_sm[dtype][v]) return GQS_ERR_NO_DEVICE;
   }
   if (n >= (1ull << 40) || nseg >= (1ull << 31)) return GQS_ERR_INVALID;
-  // the split has scratch of its own, and may leave ranges that become segments
+  // the split has scratch of its own, and may leave ranges that become segments. A plain sort and a segmented one of as many
+  // keys, even of one segment, need different tables.
   const size_t nseg_in = nseg ? nseg : 1;
-  const size_t reach = c->auto_variant[dtype] || nseg_in > 1 ? (1ull << 31) - 1 : 1ull << 21;  // the largest that use_split takes
-  const size_t m = std::min(n, reach);
-  if (use_split(c, dtype, m, nseg_in == 1)) {
-    size_t bytes = gqs::split_scratch_bytes(dtype, m, 1, true, c->num_sms);
-    if (nseg_in > 1) bytes = std::max(bytes, gqs::split_scratch_bytes(dtype, m, nseg_in, false, c->num_sms));
+  const size_t m = std::min(n, kSplitKeys), plain = std::min(m, c->auto_variant[dtype] ? kSplitKeys : kFixedMost);
+  if (m) {
+    size_t bytes = gqs::split_scratch_bytes(dtype, m, nseg_in, false, c->num_sms);
+    if (use_split(c, dtype, plain, true)) bytes = std::max(bytes, gqs::split_scratch_bytes(dtype, plain, 1, true, c->num_sms));
     gqs_status st = grow_split(c, bytes);
     if (st != GQS_OK) return st;
     if (c->split_counters.unclear()) {  // here, so that a sort that follows, or is captured, has it behind it

@@ -49,3 +49,41 @@ def test_first_small_sorts_beside_a_busy_default_stream(gpu_ctx, call, reserve):
                 got = t.cpu().numpy().view(np.uint32)
             assert np.array_equal(got, want)
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("variant", [-1, 0])
+@pytest.mark.parametrize("nseg", [1, 3])
+def test_reserve_covers_plain_and_segmented_sorts(variant, nseg):
+    """What is reserved for n keys in nseg segments sorts n keys, and fewer, as one array or as segments, and allocates nothing."""
+    torch = pytest.importorskip("torch")
+    stream = torch.cuda.current_stream().cuda_stream
+    n = 1 << 25
+    keys = torch.randint(-(1 << 31), 1 << 31, (n,), dtype=torch.int64, device="cuda").to(torch.int32)
+    order = torch.tensor([-(1 << 31)], dtype=torch.int32, device="cuda")  # signed order to unsigned
+    want = torch.sort(keys ^ order).values ^ order
+
+    def run(ctx, length, segments):
+        t = keys[:length].clone()
+        off = torch.tensor([length * i // max(segments, 1) for i in range(segments + 1)], device="cuda")
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        if segments:
+            code = ctx.sort_segments_dev("u32", t.data_ptr(), None, length, off.data_ptr(), segments, stream)
+        else:
+            code = ctx.sort_dev("u32", t.data_ptr(), None, length, stream)
+        assert code == 0
+        torch.cuda.synchronize()
+        return before - torch.cuda.mem_get_info()[0], t
+
+    with gqs_ctypes.Context(variant=variant) as ctx:
+        first = run(ctx, n, 1)  # loads the kernels
+        run(ctx, n, 0), run(ctx, 1 << 20, 0)
+        assert torch.equal(first[1], want)
+    with gqs_ctypes.Context(variant=variant) as ctx:
+        ctx.reserve("u32", n, nseg)
+        for length in (n, 1 << 20, 5000):
+            for segments in (0, 1, nseg):
+                taken, t = run(ctx, length, segments)
+                assert taken == 0, (length, segments)
+                if length == n and segments < 2:
+                    assert torch.equal(t, want)
