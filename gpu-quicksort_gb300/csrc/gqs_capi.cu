@@ -148,6 +148,7 @@ struct gqs_ctx {
   void* split_buf = nullptr;  // scratch of the top split of small sorts (gqs_split.cu)
   size_t split_bytes = 0;
   gqs::SplitCounters split_counters;  // those at its head
+  gqs::SplitRoom split_room;
   bool split_prepared[4] = {};        // per key type: its kernels may be launched on this device
   int variant[4] = {0, 0, 0, 0};  // per key type, and the internal packed pairs
   bool auto_variant[4] = {true, true, true, true};  // pick per call from the tuning table
@@ -262,8 +263,12 @@ gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, co
   if (n >= (1ull << 40) || nseg >= (1ull << 31)) return GQS_ERR_INVALID;
   const int v = c->auto_variant[dtype] ? gqs::tuned_variant(dtype, n, c->num_sms) : c->variant[dtype];
   const gqs::VariantInfo vi = gqs::variant_info(dtype, v);
-  const bool split = !check_n && use_split(c, dtype, n, offsets == nullptr);
-  const size_t split_bytes = split ? gqs::split_scratch_bytes(dtype, n, nseg, offsets == nullptr, c->num_sms) : 0;
+  bool split = !check_n && use_split(c, dtype, n, offsets == nullptr);
+  size_t split_bytes = split ? gqs::split_scratch_bytes(dtype, n, nseg, offsets == nullptr, c->num_sms) : 0;
+  if (!c->split_room.may_hold(split_bytes)) {
+    split = false;
+    split_bytes = 0;
+  }
   const size_t segs = split ? std::max(nseg, n / 4096 + 1) : nseg;
   const size_t cap = job_capacity(vi, n, segs);
   const size_t ring = ticket_ring(vi, n, segs);
@@ -308,7 +313,12 @@ gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, co
     }
     if (need_split) {
       st = grow_split(c, split_bytes);
-      if (st != GQS_OK) return st;
+      if (st == GQS_ERR_NOMEM && !capturing(stream)) {  // the persistent kernel sorts alone, in what it has
+        c->split_room.refuse(split_bytes);
+        split = false;
+      } else if (st != GQS_OK) {
+        return st;
+      }
     }
   }
   if (!dn) dn = c->pool_dn;
@@ -786,24 +796,7 @@ gqs_status gqs_reserve(gqs_ctx* c, int dtype, size_t n, size_t nseg, int with_bu
   // keys, even of one segment, need different tables.
   const size_t nseg_in = nseg ? nseg : 1;
   const size_t m = std::min(n, kSplitKeys), plain = std::min(m, c->auto_variant[dtype] ? kSplitKeys : kFixedMost);
-  if (m) {
-    size_t bytes = gqs::split_scratch_bytes(dtype, m, nseg_in, false, c->num_sms);
-    if (use_split(c, dtype, plain, true)) bytes = std::max(bytes, gqs::split_scratch_bytes(dtype, plain, 1, true, c->num_sms));
-    gqs_status st = grow_split(c, bytes);
-    if (st != GQS_OK) return st;
-    if (c->split_counters.unclear()) {  // here, so that a sort that follows, or is captured, has it behind it
-      cudaError_t e = cudaMemsetAsync(c->split_buf, 0, gqs::split_clear_bytes(), c->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-      if (e != cudaSuccess) return cuda_status(e);
-      c->split_counters.cleared();
-    }
-    if (!c->split_prepared[dtype]) {
-      const cudaError_t e = gqs::split_prepare(dtype);
-      if (e != cudaSuccess) return cuda_status(e);
-      c->split_prepared[dtype] = true;
-    }
-    nseg = std::max(nseg_in, m / 4096 + 1);
-  }
+  if (m) nseg = std::max(nseg_in, m / 4096 + 1);
   const size_t cap = job_capacity(vi, n, nseg ? nseg : 1);
   if (cap >= (1ull << 32) || ticket_ring(vi, n, nseg ? nseg : 1) > (1ull << 31)) return GQS_ERR_INVALID;
   if (c->job_cap < cap) {
@@ -833,6 +826,29 @@ gqs_status gqs_reserve(gqs_ctx* c, int dtype, size_t n, size_t nseg, int with_bu
     st = grow(&po, &c->offs_cap, (nseg_in + 1) * sizeof(uint64_t));
     c->offs = static_cast<unsigned long long*>(po);
     if (st != GQS_OK) return st;
+  }
+  if (m) {  // last: sorts can do without it
+    c->split_room.forget();
+    size_t split_bytes = gqs::split_scratch_bytes(dtype, m, nseg_in, false, c->num_sms);
+    if (use_split(c, dtype, plain, true))
+      split_bytes = std::max(split_bytes, gqs::split_scratch_bytes(dtype, plain, 1, true, c->num_sms));
+    st = grow_split(c, split_bytes);
+    if (st == GQS_ERR_NOMEM) {
+      c->split_room.refuse(1);  // no sort that relies on this call allocates
+      return GQS_OK;
+    }
+    if (st != GQS_OK) return st;
+    if (c->split_counters.unclear()) {  // here, so that a sort that follows, or is captured, has it behind it
+      cudaError_t e = cudaMemsetAsync(c->split_buf, 0, gqs::split_clear_bytes(), c->stream);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+      if (e != cudaSuccess) return cuda_status(e);
+      c->split_counters.cleared();
+    }
+    if (!c->split_prepared[dtype]) {
+      const cudaError_t e = gqs::split_prepare(dtype);
+      if (e != cudaSuccess) return cuda_status(e);
+      c->split_prepared[dtype] = true;
+    }
   }
   return GQS_OK;
 }

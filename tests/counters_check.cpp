@@ -1,7 +1,7 @@
 // Check of when a small sort's counters are cleared (gpu-quicksort_gb300/csrc/gqs_counters.h), compiled and run by
 // tests/test_counters.py on the CPU: a model of the counters beside the tracker, with launches that succeed, fail before the
 // first kernel, or fail with half of the sort enqueued, clearings that fail, captured streams, and new scratch. Every sort that
-// was enqueued as a whole must have found the counters zero. Prints "ok" and exits 0, or the violation and exits 1.
+// was enqueued as a whole must have found the counters zero. Then which scratch is asked for after a refusal. Prints "ok" and exits 0, or the violation and exits 1.
 #include <cstdio>
 #include <cstdlib>
 
@@ -53,6 +53,16 @@ int main() {
   bool again = false;
   t.enqueue<int>(false, [&] { again = true; return 0; }, [] { return 0; });
   if (again || !clears || !good) return std::printf("cleared without need\n"), 1;
+  // scratch that there was no room for
+  gqs::SplitRoom room;
+  if (!room.may_hold(0) || !room.may_hold(~(size_t)1)) return std::printf("refused at first\n"), 1;
+  room.refuse(1000);
+  room.refuse(2000);
+  if (room.may_hold(1000) || room.may_hold(2000) || !room.may_hold(999)) return std::printf("refusals not kept\n"), 1;
+  room.refuse(1);
+  if (room.may_hold(1) || !room.may_hold(0)) return std::printf("a sort without the split was refused\n"), 1;
+  room.forget();
+  if (!room.may_hold(1000)) return std::printf("a refusal was not forgotten\n"), 1;
   std::printf("ok\n");
   return 0;
 }
