@@ -256,14 +256,15 @@ bool use_split(const gqs_ctx* c, int dtype, size_t n, bool plain) {
 // caller waits for the sort next (wait_pending_locked), so the persistent kernel is launched only
 // then and only if the split has left it something.
 gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, const unsigned long long* offsets,
-                          size_t nseg, cudaStream_t stream, unsigned long long check_n = 0, bool waits = false) {
+                          size_t nseg, cudaStream_t stream, unsigned long long check_n = 0, bool waits = false,
+                          bool check_split = false) {
   const size_t es = kElemSize[dtype];
   if (!d || (reinterpret_cast<uintptr_t>(d) % es) != 0) return GQS_ERR_INVALID;
   if (dn && (reinterpret_cast<uintptr_t>(dn) % es) != 0) return GQS_ERR_INVALID;
   if (n >= (1ull << 40) || nseg >= (1ull << 31)) return GQS_ERR_INVALID;
   const int v = c->auto_variant[dtype] ? gqs::tuned_variant(dtype, n, c->num_sms) : c->variant[dtype];
   const gqs::VariantInfo vi = gqs::variant_info(dtype, v);
-  bool split = !check_n && use_split(c, dtype, n, offsets == nullptr);
+  bool split = check_split || (!check_n && use_split(c, dtype, n, offsets == nullptr));
   size_t split_bytes = split ? gqs::split_scratch_bytes(dtype, n, nseg, offsets == nullptr, c->num_sms) : 0;
   if (!c->split_room.may_hold(split_bytes)) {
     split = false;
@@ -351,7 +352,8 @@ gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, co
     gqs::SplitArgs sa{};
     sa.d = d;
     sa.dn = dn;
-    sa.n = sa.bound = n;
+    sa.n = n;
+    sa.bound = check_n ? check_n : n;
     sa.offsets = offsets;
     sa.nseg = nseg;
     sa.scratch = c->split_buf;
@@ -972,9 +974,14 @@ gqs_status gqs_selftest_bounds(gqs_ctx* c, int dtype) {
   // equal keys (0x5a bytes: an ordinary value for every key type); any keys would do
   cudaError_t e = cudaMemsetAsync(c->pool_d, 0x5a, n * es, c->stream);
   if (e != cudaSuccess) return cuda_status(e);
-  st = enqueue_locked(c, dtype, c->pool_d, nullptr, n, nullptr, 1, c->stream, n / 2);
-  if (st != GQS_OK) return st;
-  return wait_pending_locked(c);
+  // the persistent kernel by itself, then the split
+  gqs_status got[2] = {GQS_OK, GQS_OK};
+  for (int split = 0; split < 2; ++split) {
+    st = enqueue_locked(c, dtype, c->pool_d, nullptr, n, nullptr, 1, c->stream, n / 2, false, split != 0);
+    if (st != GQS_OK) return st;
+    got[split] = wait_pending_locked(c);
+  }
+  return got[0] == got[1] ? got[0] : GQS_ERR_INTERNAL;
 }
 
 gqs_status gqs_sync(gqs_ctx* c) {

@@ -296,8 +296,9 @@ __device__ __forceinline__ void level_note(Queue* q, uint32_t depth, int col, un
 }
 #endif
 
-// Debug builds (-DGQS_CHECK) test every job record, staged range and global write index
-// against the sort's bounds; a failed test records ST_BOUNDS with the site's code in
+// Debug builds (-DGQS_CHECK) test every job record, staged range and global write index, and in the
+// split (gqs_split.cu) the segments, map tables, shared-memory places and records too, against
+// the sort's bounds; a failed test records ST_BOUNDS with the site's code in
 // error_info, the access is skipped, and every role then winds down through its error path.
 // Product builds compile the tests out.
 #ifdef GQS_CHECK

@@ -32,6 +32,13 @@
 #include "gqs_device.cuh"
 #include "gqs_launch.h"
 
+// Fields and arguments that only the bounds-check build has.
+#ifdef GQS_CHECK
+#define GQS_CHECK_ONLY(...) __VA_ARGS__
+#else
+#define GQS_CHECK_ONLY(...)
+#endif
+
 namespace gqs {
 namespace {
 
@@ -134,6 +141,8 @@ struct Tables {
   unsigned long long* left;  // (start, end) of the ranges left to the quicksort
   uint32_t buckets;          // records there is room for
   uint32_t tile_keys;
+  uint32_t lefts;            // records of `left` that there is room for
+  unsigned long long n;      // every key index is below it
 };
 // The state of a small plain sort. The cursors and the count of finished CTAs are zero between sorts: the last CTA of
 // local_small leaves them so.
@@ -278,7 +287,8 @@ struct KeyMap {
   B lo, span;
   uint32_t sh, used, top, kind;
   float flo, scale;
-  __device__ __forceinline__ void load(const SegRec& r) {
+  GQS_CHECK_ONLY(Queue* q; uint32_t bins;)
+  __device__ __forceinline__ void load(const SegRec& r GQS_CHECK_ONLY(, Queue* q_)) {
     lo = (B)r.lo;
     span = (B)r.span;
     sh = r.sh;
@@ -287,7 +297,25 @@ struct KeyMap {
     kind = r.kind;
     flo = r.flo;
     scale = r.scale;
+#ifdef GQS_CHECK
+    q = q_;
+    bins = r.bins;
+    check(r.cells, r.k);
+#endif
   }
+#ifdef GQS_CHECK
+  // The map's tables are as large as was reserved for them.
+  __device__ __forceinline__ void check(uint32_t cells, uint32_t k) {
+    if (GQS_OK(used <= cells && used <= kMaxCells + kMaxSub && top < used && bins <= bin_room(k) && bins <= kBinSlots &&
+                   (kind & PART_COUNT) <= part_room(k),
+               q, 0xD203ull))
+      return;
+    lo = span = 0;
+    sh = top = kind = 0u;
+    used = 1u;
+    bins = bins < kBinSlots ? bins : kBinSlots;
+  }
+#endif
   __device__ __forceinline__ B offset(B key) const {
     const B x = (key < lo ? lo : key) - lo;
     return x < span ? x : span;
@@ -307,9 +335,20 @@ struct KeyMap {
     constexpr int kTop = sizeof(E) * 8 - 1;
     uint32_t e = tab[cell<VALUE>(key)];
     if constexpr (PARTS_) {
+#ifdef GQS_CHECK
+      for (int depth = 0; e >> kTop; ++depth) {
+        const uint32_t p = e & ((1u << kTop) - 1u);
+        if (!GQS_OK(p < (kind & PART_COUNT) && depth < 4, q, 0xD204ull)) return 0u;
+        const uint32_t at = part[p].of(key);
+        if (!GQS_OK(at < used, q, 0xD205ull)) return 0u;
+        e = tab[at];
+      }
+#else
       while (e >> kTop) e = tab[part[e & ((1u << kTop) - 1u)].of(key)];
+#endif
       if (sizeof(E) == 2 && e >> 14) e ^= 1u << 14 ^ kEqual;
     }
+    if (!GQS_OK((e & kBinMask) < bins, q, 0xD206ull)) return 0u;
     return e;
   }
   static __device__ __forceinline__ uint16_t narrow(uint32_t e) { return (uint16_t)((e & 0x3fffu) | (e >> 16 & 0xc000u)); }
@@ -781,10 +820,17 @@ __global__ void __launch_bounds__(kThreads) split_map(const BOf<T>* src, Tables 
     }
     KeyMap<T> map;
     uint32_t bins;
+    if (!GQS_OK(__ldcg(&rec->start) + __ldcg(&rec->len) <= t.n, q, 0xD207ull)) continue;
     make_map<T>(sm, src + __ldcg(&rec->start), __ldcg(&rec->len), k, s, kOver, max_sample, map, bins, [&](uint32_t b, B x) {
+      if (!GQS_OK(b < bin_room(k), q, 0xD208ull)) return;
       v.eq[bin0 + b] = 1u;
       v.value[bin0 + b] = x;
     });
+#ifdef GQS_CHECK
+    map.q = q;
+    map.bins = bins;
+    map.check(__ldcg(&rec->cells), k);
+#endif
     for (uint32_t i = tid; i < map.used; i += kThreads) v.cell[cell0 + i] = sm.tab[i];
     Part<B>* const out = static_cast<Part<B>*>(v.part) + bin0 / 4u;
     for (uint32_t i = tid; i < (map.kind & PART_COUNT); i += kThreads) out[i] = sm.part[i];
@@ -818,7 +864,7 @@ __device__ __forceinline__ uint32_t find_segment(const SegRec* seg, uint32_t nse
 // Every key's range, counted: reads the keys once. Bound by shared memory (a cell and a count each, seven wavefronts a row of 32)
 // 62 to 70 % of the rate, half the copy bandwidth: 2^25 u32 in 35 to 40 us. Three CTAs on an SM hide its loads, eight under way a thread.
 template <class T>
-__global__ void __launch_bounds__(kThreads, 3) split_count(const BOf<T>* src, Tables t, Level v, const Queue* q) {
+__global__ void __launch_bounds__(kThreads, 3) split_count(const BOf<T>* src, Tables t, Level v, Queue* q) {
   using B = BOf<T>;
   __shared__ uint32_t tab[kMaxCells + kMaxSub];
   __shared__ uint32_t cnt[kBinSlots];
@@ -839,7 +885,7 @@ __global__ void __launch_bounds__(kThreads, 3) split_count(const BOf<T>* src, Ta
     const uint32_t seg_tiles = (r.len + tile_keys - 1u) / tile_keys;
     const uint32_t end = r.tile0 + seg_tiles < t1 ? r.tile0 + seg_tiles : t1;
     KeyMap<T> map;
-    map.load(r);
+    map.load(r GQS_CHECK_ONLY(, q));
     __syncthreads();
     for (uint32_t i = tid; i < map.used; i += kThreads) tab[i] = v.cell[r.cell0 + i];
     for (uint32_t i = tid; i < (map.kind & PART_COUNT); i += kThreads) part[i] = static_cast<const Part<B>*>(v.part)[r.bin0 / 4u + i];
@@ -933,6 +979,7 @@ __global__ void __launch_bounds__(kThreads) split_starts(Tables t, Level v, Leve
       uint32_t first = 0u;
       if (lane == 31 && inc) first = atomicAdd(&t.ctl->buckets, inc);
       first = __shfl_sync(0xffffffffu, first, 31) + inc - recs;
+      if (recs && !GQS_OK(first + recs <= t.buckets && start + c[i] <= r.start + r.len, q, 0xD209ull)) continue;
       for (uint32_t j = 0; j < recs; ++j) {
         const uint32_t off = j * kCopyChunk;
         t.bucket[first + j] = eq ? Bucket{start + off, c[i] - off < kCopyChunk ? c[i] - off : kCopyChunk, EQUAL, v.value[r.bin0 + b]}
@@ -1048,12 +1095,16 @@ __device__ __forceinline__ void scatter_tile(TileSmem<BOf<T>>& sm, const KeyMap<
     for (int j = 0; j < ROWS; ++j)
       if (at[j] != kLeft) {
         const uint32_t i = sm.cnt[at[j] >> 16] + (at[j] & 0xffffu);
+        if (!GQS_OK(i < here, map.q, 0xD20Aull)) continue;
         sm.keys[i] = key[j];
         sm.bin[i] = (uint16_t)(at[j] >> 16);  // cheaper than to find it again
       }
   } else if (full && !runs) {
 #pragma unroll
-    for (int j = 0; j < ROWS; ++j) sm.keys[atomicAdd(&sm.cnt[range_of(j)], 1u)] = key[j];
+    for (int j = 0; j < ROWS; ++j) {
+      const uint32_t i = atomicAdd(&sm.cnt[range_of(j)], 1u);
+      if (GQS_OK(i < here, map.q, 0xD20Aull)) sm.keys[i] = key[j];
+    }
   } else if (full) {
 #pragma unroll
     for (int j = 0; j < ROWS; ++j) {
@@ -1065,12 +1116,15 @@ __device__ __forceinline__ void scatter_tile(TileSmem<BOf<T>>& sm, const KeyMap<
         if (lane == 0) i = atomicAdd(&sm.cnt[b], 32u);
         i = __shfl_sync(0xffffffffu, i, 0) + lane;
       }
-      sm.keys[i] = key[j];
+      if (GQS_OK(i < here, map.q, 0xD20Aull)) sm.keys[i] = key[j];
     }
   } else {
 #pragma unroll
     for (int j = 0; j < ROWS; ++j)
-      if (range_of(j) != kLeft) sm.keys[atomicAdd(&sm.cnt[range_of(j)], 1u)] = key[j];
+      if (range_of(j) != kLeft) {
+        const uint32_t i = atomicAdd(&sm.cnt[range_of(j)], 1u);
+        if (GQS_OK(i < here, map.q, 0xD20Aull)) sm.keys[i] = key[j];
+      }
   }
   if (b0 < bins) sm.gbase[b0] = base0 - ex0;
   between();
@@ -1150,7 +1204,7 @@ __global__ void __launch_bounds__(kThreads, kTileCtas) split_scatter(const BOf<T
   for (uint32_t tile = t0; tile < t1; ++tile) {
     if (fresh) {
       const SegRec* const r = v.seg + s;
-      map.load(*r);
+      map.load(*r GQS_CHECK_ONLY(, q));
       bins = r->bins;
       cursor = v.bin + r->bin0;
       out = dst + start;
@@ -1168,10 +1222,14 @@ __global__ void __launch_bounds__(kThreads, kTileCtas) split_scatter(const BOf<T
     const uint32_t here = len;
     B* const to = out;
     uint32_t* const cur = cursor;
+    GQS_CHECK_ONLY(const uint32_t keys = seg_len;)
     by_kind<T>(map.kind, [&]<bool VALUE, bool PARTS_>() {
       scatter_tile<T, VALUE, PARTS_, false>(
           sm.tile, map, sm.tab, sm.part, bins, key, here, [&](uint32_t b, uint32_t c) { return atomicAdd(cur + b, c); },
-          [&] { advance(tile); }, [&](uint32_t, uint32_t at, B k) { to[at] = KeyOps<T>::raw(k); });
+          [&] { advance(tile); },
+          [&](uint32_t, uint32_t at, B k) {
+            if (GQS_OK(at < keys, q, 0xD20Bull)) to[at] = KeyOps<T>::raw(k);
+          });
     });
   }
   if (tid == 0) atomicAdd(&q->chunks, (unsigned long long)(t1 - t0));
@@ -1211,11 +1269,17 @@ __global__ void __cluster_dims__(CL) __launch_bounds__(kThreads, kTileCtas) spli
   if (blockIdx.x == 0) clear(st->eq, bin_room(k) * 4);
   if (blockIdx.x == 1) clear(q, sizeof(Queue));
   make_map<T, CL>(sm.map, src, n, k, 0u, kSmallOver, Sizes<B>::kSmallSample, map, bins, [&](uint32_t b, B x) {
-    if (blockIdx.x == 0) {
+    if (blockIdx.x == 0 && GQS_OK(b < bin_room(k), q, 0xD208ull)) {
       st->eq[b] = 1u;
       st->value[b] = x;
     }
   });
+#ifdef GQS_CHECK
+  map.q = q;
+  map.bins = bins;
+  map.check(cell_count(k) + sub_room(k), k);
+  bins = map.bins;
+#endif
   if (blockIdx.x == 0 && tid == 0) {
     st->bins = bins;
     st->left = 0ull;
@@ -1246,7 +1310,7 @@ __global__ void __cluster_dims__(CL) __launch_bounds__(kThreads, kTileCtas) spli
           [&](uint32_t b, uint32_t at, B x) {
             // keys past the room are dropped: local_small sees that the range is too long and leaves the sort (its keys are
             // still in d) to the persistent kernel
-            if (at < LT) area[(size_t)b * LT + at] = KeyOps<T>::raw(x);
+            if (at < LT && GQS_OK(b < bin_room(k), q, 0xD20Cull)) area[(size_t)b * LT + at] = KeyOps<T>::raw(x);
           });
     });
     __syncthreads();
@@ -1314,9 +1378,10 @@ struct LocalSmem {
   B wmin[Sizes<B>::kSortThreads / 32], wmax[Sizes<B>::kSortThreads / 32];
   uint32_t wsum[Sizes<B>::kSortThreads / 32];
   uint32_t most;
-  uint32_t todos;                                           // bins for a warp each
-  uint16_t todo[Sizes<B>::kLocal / (Sizes<B>::kShortBin + 1) + 2];
-  uint32_t bigs, big[Sizes<B>::kLocal / (kWarpBin + 1) + 1];  // bins for the CTA, later: (first key << 16) | keys
+  static constexpr uint32_t kTodos = Sizes<B>::kLocal / (Sizes<B>::kShortBin + 1) + 2, kBigs = Sizes<B>::kLocal / (kWarpBin + 1) + 1;
+  uint32_t todos;            // bins for a warp each
+  uint16_t todo[kTodos];
+  uint32_t bigs, big[kBigs];  // bins for the CTA, later: (first key << 16) | keys
   static constexpr uint32_t V = 16 / sizeof(B), kPieces = Sizes<B>::kBlock / V;  // keys of a piece, pieces of a block
   static __device__ __forceinline__ uint32_t slot(uint32_t i) { return i ^ ((i / V >> 3 & (kPieces - 1u)) * V); }
   __device__ __forceinline__ uint4* piece(uint32_t b, uint32_t i) {
@@ -1430,7 +1495,7 @@ struct BinMap {
 // networks over neighbouring blocks finish the order without knowing the bins.
 template <class T, class Between>
 __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[Sizes<BOf<T>>::kLocalRows], uint32_t len, BOf<T>* dst,
-                                          uint32_t off, bool first, Between&& between) {
+                                          uint32_t off, bool first, Queue* q, Between&& between) {
   using B = BOf<T>;
   using S = LocalSmem<B>;
   constexpr int ROWS = Sizes<B>::kLocalRows;
@@ -1473,7 +1538,7 @@ __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[S
     for_rows<ROWS, NT>(len, [&](int j) {
       key[j] = near.in(key[j]);
       const uint32_t b = map.template of<VALUE>(key[j]);
-      atomicAdd(&sm.cur[b >> 1], b & 1u ? 0x10000u : 1u);
+      if (GQS_OK(b < bins, q, 0xD20Dull)) atomicAdd(&sm.cur[b >> 1], b & 1u ? 0x10000u : 1u);
     });
   };
   if (kFloating<T> && map.by_value) count.template operator()<kFloating<T>>();
@@ -1531,7 +1596,9 @@ __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[S
   auto place = [&]<bool VALUE>() {
     for_rows<ROWS, NT>(len, [&](int j) {
       const uint32_t b = map.template of<VALUE>(key[j]);
+      if (!GQS_OK(b < bins, q, 0xD20Dull)) return;
       const uint32_t old = atomicAdd(&sm.cur[b >> 1], b & 1u ? 0x10000u : 1u);
+      if (!GQS_OK((b & 1u ? old >> 16 : old & 0xffffu) < len, q, 0xD20Eull)) return;
       sm.keys[S::slot(b & 1u ? old >> 16 : old & 0xffffu)] = key[j];
     });
   };
@@ -1559,12 +1626,15 @@ __device__ __forceinline__ void sort_bins(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[S
       const uint32_t b = map.any(k), s = first_of(b);
       if (end_of(b) - s > kShortBin && k != sm.keys[S::slot(s)] && !mark(b)) {
         const uint32_t n = end_of(b) - s;
-        if (n <= kWarpBin) sm.todo[atomicAdd(&sm.todos, 1u)] = (uint16_t)b;
-        else sm.big[atomicAdd(&sm.bigs, 1u)] = ((off + s) << 16) | n;
+        if (!GQS_OK(s + n <= len, q, 0xD20Full)) continue;
+        const uint32_t to = atomicAdd(n <= kWarpBin ? &sm.todos : &sm.bigs, 1u);
+        if (!GQS_OK(to < (n <= kWarpBin ? S::kTodos : S::kBigs), q, 0xD20Full)) continue;
+        if (n <= kWarpBin) sm.todo[to] = (uint16_t)b;
+        else sm.big[to] = ((off + s) << 16) | n;
       }
     }
     __syncthreads();
-    const uint32_t m = sm.todos;
+    const uint32_t m = GQS_OK(sm.todos <= S::kTodos, q, 0xD20Full) ? sm.todos : 0u;
     for (uint32_t t = warp; t < m; t += NT / 32) {
       const uint32_t b = sm.todo[t], s = first_of(b), n = end_of(b) - s;
       auto sort_bin = [&]<int R>() {
@@ -1641,23 +1711,24 @@ __device__ __forceinline__ void load_range(const B* p, uint32_t len, B (&raw)[Si
 // Returns whether there were any (the keys that between() loaded are then lost).
 template <class T, class Between>
 __device__ __forceinline__ bool sort_range(LocalSmem<BOf<T>>& sm, BOf<T> (&key)[Sizes<BOf<T>>::kLocalRows], uint32_t len, BOf<T>* dst,
-                                           Between&& between) {
+                                           Queue* q, Between&& between) {
   using B = BOf<T>;
   if (threadIdx.x == 0) sm.bigs = 0u;
-  sort_bins<T>(sm, key, len, dst, 0u, true, between);
+  sort_bins<T>(sm, key, len, dst, 0u, true, q, between);
   if (sm.most <= kWarpBin) return false;
   bool again = false;
   while (true) {
     __syncthreads();  // every thread has read what changes below, and sees the keys in dst
-    const uint32_t m = sm.bigs;
+    const uint32_t m = GQS_OK(sm.bigs <= LocalSmem<B>::kBigs, q, 0xD20Full) ? sm.bigs : 0u;
     if (!m) return again;
     again = true;
     const uint32_t e = sm.big[m - 1u];
     __syncthreads();
     if (threadIdx.x == 0) sm.bigs = m - 1u;
+    if (!GQS_OK((e >> 16) + (e & 0xffffu) <= len, q, 0xD210ull)) continue;
     load_range<B>(dst + (e >> 16), e & 0xffffu, key);
     for_rows<Sizes<B>::kLocalRows, Sizes<B>::kSortThreads>(e & 0xffffu, [&](int j) { key[j] = KeyOps<T>::key(key[j]); });
-    sort_bins<T>(sm, key, e & 0xffffu, dst, e >> 16, false, [] {});
+    sort_bins<T>(sm, key, e & 0xffffu, dst, e >> 16, false, q, [] {});
   }
 }
 
@@ -1740,6 +1811,7 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
         moved += len;
       } else if (tid == 0) {
         const unsigned long long to = atomicAdd(&t.ctl->leftovers, 1ull);
+        if (!GQS_OK(to < t.lefts, q, 0xD211ull)) break;
         t.left[2 * to] = bk.start;
         t.left[2 * to + 1] = bk.start + len;
         atomicAdd(&q->left, 1u);
@@ -1754,7 +1826,7 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
 #endif
     load_range<B>(src, len, key);
     if (!KeyOps<T>::kIdentity) for_rows<ROWS, NT>(len, [&](int j) { key[j] = KeyOps<T>::key(key[j]); });
-    sort_range<T>(sm, key, len, dst, [&] {
+    sort_range<T>(sm, key, len, dst, q, [&] {
       if (more) fetch(coming);
     });
   }
@@ -1798,7 +1870,7 @@ __device__ __forceinline__ void leave_small(Small* st, uint32_t bins, uint32_t t
 // all ranges in one round, its turn's answer is not waited for, and long ranges of equal keys are shared by all CTAs.
 // The ranges of a small sort: their starts are the scan of their counts, which every CTA makes for itself.
 template <class T>
-__global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<BOf<T>>::kSortCtas) local_small(BOf<T>* d, const BOf<T>* area, uint32_t n, Small* st, Queue* q) {
+__global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<BOf<T>>::kSortCtas) local_small(BOf<T>* d, const BOf<T>* area, uint32_t n, unsigned long long bound, Small* st, Queue* q) {
   using B = BOf<T>;
   constexpr int ROWS = Sizes<B>::kLocalRows;
   constexpr uint32_t NT = Sizes<B>::kSortThreads, LT = Sizes<B>::kLocal;
@@ -1849,8 +1921,12 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
 #pragma unroll
   for (uint32_t i = 0; i < R; ++i) {
     const uint32_t b = tid * per + i;
-    if (i < per && b < bins && b % gridDim.x == blockIdx.x) sm.own[b / gridDim.x] = Extent{b, at, c[i], equal >> i & 1u};
-    if (c[i] > kCopyChunk) sm.fill[atomicAdd(&sm.fills, 1u)] = Extent{b, at, c[i], 1u};
+    if (i < per && b < bins && b % gridDim.x == blockIdx.x && GQS_OK(b / gridDim.x < kOwnRanges, q, 0xD212ull))
+      sm.own[b / gridDim.x] = Extent{b, at, c[i], equal >> i & 1u};
+    if (c[i] > kCopyChunk) {
+      const uint32_t to = atomicAdd(&sm.fills, 1u);
+      if (GQS_OK(to < sizeof(sm.fill) / sizeof(sm.fill[0]), q, 0xD213ull)) sm.fill[to] = Extent{b, at, c[i], 1u};
+    }
     at += c[i];
   }
   __syncthreads();
@@ -1858,7 +1934,7 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
   uint32_t jobs = 0u;
   for (uint32_t o = 0; o * gridDim.x + blockIdx.x < bins; ++o) {
     const uint32_t b = sm.own[o].bin, start = sm.own[o].start, len = sm.own[o].len;
-    if (!len || !GQS_OK(start + len <= n, q, 0xD202ull)) continue;
+    if (!len || !GQS_OK((unsigned long long)start + len <= bound, q, 0xD202ull)) continue;
     if (sm.own[o].equal) {
       if (len <= kCopyChunk) {
         const B x = KeyOps<T>::raw((B)st->value[b]);
@@ -1875,11 +1951,12 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
     B key[ROWS];
     load_range<B>(area + (size_t)b * LT, len, key);
     if (!KeyOps<T>::kIdentity) for_rows<ROWS, NT>(len, [&](int j) { key[j] = KeyOps<T>::key(key[j]); });
-    sort_range<T>(sm.local, key, len, d + start, [] {});
+    sort_range<T>(sm.local, key, len, d + start, q, [] {});
   }
   // long ranges of equal keys: every CTA writes a part of each
-  for (uint32_t f = 0; f < sm.fills; ++f) {
+  for (uint32_t f = 0; f < sm.fills GQS_CHECK_ONLY(&& f < sizeof(sm.fill) / sizeof(sm.fill[0])); ++f) {
     const uint32_t b = sm.fill[f].bin, start = sm.fill[f].start, len = sm.fill[f].len;
+    if (!GQS_OK((unsigned long long)start + len <= bound, q, 0xD202ull)) continue;
     const B x = KeyOps<T>::raw((B)st->value[b]);
     const uint32_t i0 = (uint32_t)((unsigned long long)len * blockIdx.x / gridDim.x);
     const uint32_t i1 = (uint32_t)((unsigned long long)len * (blockIdx.x + 1u) / gridDim.x);
@@ -1955,10 +2032,10 @@ struct Layout {
                  p + part_at[l],
                  (uint32_t)segs[l], (uint32_t)bins[l], (uint32_t)cells[l], (uint32_t)l};
   }
-  Tables tables(void* scratch, uint32_t tile_keys) const {
+  Tables tables(void* scratch, uint32_t tile_keys, unsigned long long bound) const {
     char* p = static_cast<char*>(scratch);
     return Tables{reinterpret_cast<Ctl*>(p + ctl_at), reinterpret_cast<Bucket*>(p + bucket_at),
-                  reinterpret_cast<unsigned long long*>(p + left_at), (uint32_t)buckets, tile_keys};
+                  reinterpret_cast<unsigned long long*>(p + left_at), (uint32_t)buckets, tile_keys, (uint32_t)left, bound};
   }
 };
 
@@ -2013,7 +2090,7 @@ cudaError_t launch_t(const SplitArgs& a, SplitResult* out) {
       go(split_small<T, 1>, tiles, kThreads, sizeof(SmallSmem<B>), (const B*)d, area, n, k, st, tile_keys, a.q);
     }
     const uint32_t ranges = bin_room(k), few = sms * Sizes<B>::kSortCtas, enough = (ranges + kOwnRanges - 1u) / kOwnRanges;
-    go(local_small<T>, few > ranges ? ranges : few > enough ? few : enough, Sizes<B>::kSortThreads, sizeof(SmallSortSmem<B>), d, (const B*)area, n, st, a.q);
+    go(local_small<T>, few > ranges ? ranges : few > enough ? few : enough, Sizes<B>::kSortThreads, sizeof(SmallSortSmem<B>), d, (const B*)area, n, a.bound, st, a.q);
     out->table = reinterpret_cast<const unsigned long long*>(base + lay.small_at + offsetof(Small, table));
     out->count = reinterpret_cast<const unsigned long long*>(base + lay.small_at + offsetof(Small, left));
     out->most = 1u;
@@ -2024,7 +2101,7 @@ cudaError_t launch_t(const SplitArgs& a, SplitResult* out) {
   // larger ranges a level write longer runs.
   const uint32_t levels = a.n > (size_t)kMaxBins * Sizes<B>::kTarget || (plain && a.n > (1u << 21)) ? 2u : a.n > Sizes<B>::kLocal ? 1u : 0u;
   while (tile_keys > 4u * kThreads && a.n / tile_keys < 2u * sms) tile_keys -= 2u * kThreads;
-  const Tables t = lay.tables(a.scratch, tile_keys);
+  const Tables t = lay.tables(a.scratch, tile_keys, a.bound);
   const Level lv[2] = {lay.level(a.scratch, 0), lay.level(a.scratch, 1)};
   if (!plain) {  // the first kernel of a plain sort clears them
     e = cudaMemsetAsync(a.q, 0, sizeof(Queue), s);
@@ -2044,7 +2121,7 @@ cudaError_t launch_t(const SplitArgs& a, SplitResult* out) {
     const uint32_t tiles = (uint32_t)(a.n / tile_keys + lay.segs[l]);
     const uint32_t sample = plain && !l ? Sizes<B>::kMaxSample : Sizes<B>::kMaxSample2;
     go(split_map<T>, gs, kThreads, sizeof(MapSmem<B>) + sample * sizeof(B), src, t, lv[l], plain && !l ? (uint32_t)a.n : 0u, levels, sample, a.q);
-    go(split_count<T>, least(sms * 3u, tiles), kThreads, 0, src, t, lv[l], (const Queue*)a.q);
+    go(split_count<T>, least(sms * 3u, tiles), kThreads, 0, src, t, lv[l], a.q);
     go(split_starts<T>, gs, kThreads, 0, t, lv[l], lv[1], levels, a.q);
     go(split_scatter<T>, least(sms * kTileCtas, tiles), kThreads, sizeof(ScatterSmem<B>), src, dst, t, lv[l], a.q);
   }

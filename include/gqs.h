@@ -276,8 +276,9 @@ uint64_t gqs_srv_now_ns(void);
 gqs_status gqs_selftest_stalled_queue(gqs_ctx* ctx, int dtype, uint32_t timeout_ms);
 
 /* Self-test of the bounds checks of a -DGQS_CHECK build (libgqs_check.so): sorts 2^16 keys of
- * type `dtype` in the context's pool while telling the kernel that key indices end at 2^15, so
- * the first job already lies outside the bound. A check build reports GQS_ERR_BOUNDS without
+ * type `dtype` in the context's pool while telling the kernels that key indices end at 2^15, once
+ * by the persistent kernel, whose first job already lies outside the bound, and once by the split,
+ * one of whose ranges does. A check build reports GQS_ERR_BOUNDS without
  * touching anything past the bound; the product build, whose checks are compiled out, sorts the
  * keys and returns GQS_OK. Every access stays inside the 2^16-key buffers either way. */
 gqs_status gqs_selftest_bounds(gqs_ctx* ctx, int dtype);
