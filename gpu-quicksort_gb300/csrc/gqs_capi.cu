@@ -361,14 +361,13 @@ gqs_status enqueue_locked(gqs_ctx* c, int dtype, void* d, void* dn, size_t n, co
     sa.sms = c->num_sms;
     sa.stream = stream;
     gqs::SplitResult left{};
-    const bool captured = capturing(stream);
     e = c->split_counters.enqueue<cudaError_t>(
-        captured, [&] { return cudaMemsetAsync(c->split_buf, 0, gqs::split_clear_bytes(), stream); },
+        [&] { return capturing(stream); }, [&] { return cudaMemsetAsync(c->split_buf, 0, gqs::split_clear_bytes(), stream); },
         [&] { return gqs::split_launch(dtype, sa, &left); });
     if (e != cudaSuccess) {
       const gqs_status failed = cuda_status(e);
       // the next sort, on whatever stream, finds none of this one's kernels still running
-      if (!captured) cudaStreamSynchronize(stream);
+      if (!capturing(stream)) cudaStreamSynchronize(stream);
       (void)cudaGetLastError();
       return failed;
     }

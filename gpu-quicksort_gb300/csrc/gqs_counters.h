@@ -27,9 +27,10 @@ class SplitCounters {
   void cleared() { unclear_ = false; }
 
   // Enqueues one sort with launch(), behind clear() if the counters may not be zero; both return a status, S{} for success. In a
-  // stream that is being captured (`captured`) neither has run when this returns: the graph clears them for itself.
-  template <class S, class Clear, class Launch>
-  S enqueue(bool captured, Clear&& clear, Launch&& launch) {
+  // stream that is being captured (captured(), asked only after a clearing) neither has run when this returns: the graph clears
+  // them for itself.
+  template <class S, class Captured, class Clear, class Launch>
+  S enqueue(Captured&& captured, Clear&& clear, Launch&& launch) {
     const bool was = unclear_;
     if (was) {
       const S e = clear();
@@ -37,7 +38,7 @@ class SplitCounters {
     }
     unclear_ = true;
     const S e = launch();
-    if (e == S{}) unclear_ = was && captured;
+    if (e == S{}) unclear_ = was && captured();
     return e;
   }
 };

@@ -1902,19 +1902,18 @@ __global__ void __launch_bounds__((int)Sizes<BOf<T>>::kSortThreads, (int)Sizes<B
   }
   full = __syncthreads_or(full);  // (and every thread has its counts)
   const uint32_t turn = tid == 0 ? take_turn(st) : 0u;
-  if (full) {
-    if (blockIdx.x == 0 && tid == 0) {  // d is as it was: all of it is left to the persistent kernel
-      st->table[0] = 0ull;
-      st->table[1] = n;
-      st->left = 1ull;
-      q->left = 1u;
-    }
-    leave_small(st, bins, turn);
-    return;
-  }
   uint32_t at = block_scan<NT>(sum, sm.wsum, total);
-  if (total != n) {  // the counters were not zero when the sort began: no start below can be relied on
-    if (blockIdx.x == 0 && tid == 0) set_error(q, ST_INTERNAL, total);
+  if (full || total != n) {
+    if (blockIdx.x == 0 && tid == 0) {
+      if (full) {  // d is as it was: all of it is left to the persistent kernel
+        st->table[0] = 0ull;
+        st->table[1] = n;
+        st->left = 1ull;
+        q->left = 1u;
+      } else {  // the counters were not zero when the sort began: no start below can be relied on
+        set_error(q, ST_INTERNAL, total);
+      }
+    }
     leave_small(st, bins, turn);
     return;
   }

@@ -25,7 +25,7 @@ int main() {
     bool graph_clears = false, found_zero = false;
     const bool unclear = t.unclear();
     const int e = t.enqueue<int>(
-        captured,
+        [&] { return captured; },
         [&] {
           ++clears;
           if (clear_fails) return 2;
@@ -49,9 +49,9 @@ int main() {
     good += e == 0;
   }
   // a sort that follows a good one clears nothing
-  t.enqueue<int>(false, [&] { zero = true; return 0; }, [] { return 0; });
+  t.enqueue<int>([] { return false; }, [&] { zero = true; return 0; }, [] { return 0; });
   bool again = false;
-  t.enqueue<int>(false, [&] { again = true; return 0; }, [] { return 0; });
+  t.enqueue<int>([] { return false; }, [&] { again = true; return 0; }, [] { return 0; });
   if (again || !clears || !good) return std::printf("cleared without need\n"), 1;
   // scratch that there was no room for
   gqs::SplitRoom room;
