@@ -1,10 +1,11 @@
 // Batched segmented sort as one replayable CUDA graph (gqs_batch_* in include/gqs.h), and the
-// autotuner that picks its kernel variant.
+// autotuner that picks the variant of its persistent kernel.
 //
 // The reference sorts one array per call and drives every partition level from the host
 // (GPU-Quicksort_Full_SYCL/QuicksortMain.cpp:835-906). A batch sorts thousands of independent
-// arrays in one persistent launch: the seed kernel turns the segment table into root jobs and
-// the persistent kernel drains all of them from one device queue. Everything one batch needs
+// arrays in one chain of launches: the split (gqs_split.cu), then the seed kernel, which turns what
+// the split left into root jobs, and the persistent kernel, which drains them from one device
+// queue. From 2^31 keys on, those two sort the segments alone. Everything one batch needs
 // is captured once per (key type, variant) as a CUDA graph, so a batch costs one
 // cudaGraphLaunch on the host.
 #include <cuda_runtime.h>

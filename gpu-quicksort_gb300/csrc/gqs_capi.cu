@@ -3,8 +3,8 @@
 // Host-side replacement for the reference's GPUQSort<T> driver
 // (GPU-Quicksort_Full_SYCL/QuicksortMain.cpp:835-906). The reference rebuilds its records on the
 // host and reads results back after every partition level (QuicksortMain.cpp:858-899); here one
-// seed launch and one persistent launch sort the whole array, and the host only reads a small
-// status block at the end.
+// chain of launches sorts the whole array (the split, and for what it leaves a seed and a persistent
+// kernel), and the host only reads a small status block at the end.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -145,7 +145,7 @@ struct gqs_ctx {
   unsigned long long last_lvl[gqs::kLevels][6] = {};  // per-level rows of the last sort
   unsigned long long last_lvl_start = 0;
 #endif
-  void* split_buf = nullptr;  // scratch of the top split of small sorts (gqs_split.cu)
+  void* split_buf = nullptr;  // scratch of the split (gqs_split.cu)
   size_t split_bytes = 0;
   gqs::SplitCounters split_counters;  // those at its head
   gqs::SplitRoom split_room;

@@ -657,7 +657,7 @@ __device__ unsigned long long dispatch_range(const SortArgs<typename C::T>& a, u
 
 // Segment i is [offsets[i], offsets[i+1]) or, with `pairs`, [offsets[2i], offsets[2i+1]) (the
 // segments then need not be adjacent); without offsets, the one segment [0, n). Every segment
-// must lie in [0, n). The keys are in d, or with `from_dn` in dn (the buckets of a top split);
+// must lie in [0, n). The keys are in d, or with `from_dn` in dn (ranges that the split left);
 // either way the sorted keys end in d.
 template <class C>
 __global__ void __launch_bounds__(256) seed_kernel(SortArgs<typename C::T> a, const unsigned long long* offsets,
@@ -685,7 +685,7 @@ __global__ void __launch_bounds__(256) seed_kernel(SortArgs<typename C::T> a, co
   if (e == s) return;
   if (lane == 0) atomicAdd(&a.q->total, e - s);
   unsigned long long tiny = 0;
-  // the buckets of a top split are its children: depth 1
+  // ranges of the split's first level are its children: depth 1
   const unsigned long long placed = dispatch_range<C>(a, from_dn ? 0u : 1u, s, e, from_dn ? 1u : 0u, tiny);
   if (lane == 0) {
     if (placed) atomicAdd(&a.q->done, placed);

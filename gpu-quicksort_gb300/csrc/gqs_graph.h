@@ -3,7 +3,7 @@
 // (gqs_serve.cu).
 //
 // The graph holds the whole sort: copy of the segment table from pinned host memory, clearing
-// of the status block and ticket ring, the seed kernel, the persistent kernel, and the copy of
+// of the ticket ring and status block, the split, the seed kernel, the persistent kernel, and the copy of
 // the status block back to pinned host memory. The segment count is the table's first word,
 // so one graph replays batches of any shape up to the capacities it was built for; replay is
 // one cudaGraphLaunch.

@@ -1,7 +1,10 @@
 // The fastest kernel variant per (SM count, key type, size class), the counterpart of the
 // reference's size-dependent launch parameters (optp, GPU-Quicksort_Full_SYCL/QuicksortMain.cpp:
 // 831-833). A context created with variant -1 looks up every sort here by the device's SM count
-// and ceil(log2 n); rows are written by gpu-quicksort_gb300/tune_variants.py from timed sorts.
+// and ceil(log2 n); rows are written by gpu-quicksort_gb300/tune_variants.py from timed sorts. The
+// variant sorts what the split (gqs_split.cu) leaves over, and by itself sorts of 2^31 keys and more.
+// Classes 15 to 21: timed when a split into 256 ranges stood in front of the kernel; the split that
+// has taken its place sorts those sizes whatever the variant, so they cannot be timed again.
 // Rows below: NVIDIA GB300, 152 SMs, median of 7 sorts per variant and size.
 #pragma once
 

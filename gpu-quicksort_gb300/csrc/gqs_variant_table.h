@@ -2,7 +2,8 @@
 // sort switch), chunk keys (keys per consumer thread = chunk / (32 * consumer warps)),
 // stages, keys per lane of the largest register sort>.
 // The build compiles gqs_variant_tu.cu once per entry; a context picks one per call from the
-// tuning table (gqs_tuning.h) by key type and size, and the batch autotuner times them all.
+// tuning table (gqs_tuning.h) by key type and size, and the batch autotuner times them all. They are
+// of the persistent kernel, which sorts what the split (gqs_split.cu) leaves, and the longest sorts.
 // Variant 6 halves variant 0's chunk, so that small sorts spread each level over more CTAs.
 #pragma once
 #define GQS_VARIANTS_U32(X)                                  \

@@ -6,7 +6,9 @@ For each key type (u32, f32, f64 keys; u64 for the packed words of the pair sort
 HBM, the L2 flushed before each sort of less than 256 MiB): `reps` timed sorts after two warm-up
 sorts, median kept by CUDA events around the call on its stream. The fastest variant of each
 (key type, size) becomes a row keyed by the GPU's SM count. A context created with variant -1
-then uses it for every sort whose size rounds up to that class. Run on the target GPU from the
+then uses it for every sort whose size rounds up to that class, for what the split leaves over.
+Classes 15 to 21 get no row: the split sorts those sizes whatever the variant, and the nearest
+class stands for them. Run on the target GPU from the
 repository root, then rebuild:
 
     python gpu-quicksort_gb300/tune_variants.py [--lo 10] [--hi 29] [--reps 7] [--json out.json]
@@ -76,6 +78,8 @@ def main() -> None:
         nvar = len(gqs_ctypes.variants("f64" if dtype == "u64" else dtype))
         hi = min(args.hi, 28) if dtype in ("f64", "u64") else args.hi
         for lg in range(args.lo, hi + 1):
+            if 15 <= lg <= 21:
+                continue
             n = 1 << lg
             if dtype == "u64":  # pair sort: u32 keys, u32 values 0..n-1 (packed into u64 words)
                 keys = gqs_ctypes.generate("u32", "uniform", 20260501 + lg, n)
@@ -102,7 +106,8 @@ def main() -> None:
     text = f"""// The fastest kernel variant per (SM count, key type, size class), the counterpart of the
 // reference's size-dependent launch parameters (optp, GPU-Quicksort_Full_SYCL/QuicksortMain.cpp:
 // 831-833). A context created with variant -1 looks up every sort here by the device's SM count
-// and ceil(log2 n); rows are written by gpu-quicksort_gb300/tune_variants.py from timed sorts.
+// and ceil(log2 n); rows are written by gpu-quicksort_gb300/tune_variants.py from timed sorts. The
+// variant sorts what the split (gqs_split.cu) leaves over, and by itself sorts of 2^31 keys and more.
 // Rows below: {props.name}, {sms} SMs, median of {args.reps} sorts per variant and size.
 #pragma once
 

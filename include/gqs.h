@@ -49,7 +49,8 @@ typedef enum gqs_status {
 typedef enum gqs_dtype { GQS_U32 = 0, GQS_F32 = 1, GQS_F64 = 2 } gqs_dtype;
 
 typedef struct gqs_config {
-  int32_t variant;     /* -1: per sort, the tuned variant for its key type and size; else fixed */
+  int32_t variant;     /* of the persistent kernel: -1, per sort, the tuned one for its key type and
+                          size; else fixed (see gqs_variant_count for what it sorts) */
   uint32_t timeout_ms; /* device-side no-progress limit for bounded waits; 0 means 4000 */
   uint32_t sync;       /* 1 (default): *_dev calls wait for the stream and return the device status */
   uint32_t timing;     /* 1: time the sort's kernels with CUDA events (gqs_stats.kernel_ms) */
@@ -65,7 +66,9 @@ typedef struct gqs_stats {
   uint64_t chunks;     /* partition chunks processed */
   uint64_t algo_bytes; /* key bytes * 2 * (part_keys + local_keys + tiny_keys) */
   uint32_t part_jobs, local_jobs, fill_chunks, max_depth;
-  uint32_t status, variant, grid, threads;
+  uint32_t status;
+  uint32_t variant, grid, threads; /* of the persistent kernel chosen for the sort; most often the
+                                      split leaves it nothing (gqs_last_phases is zero then) */
   double kernel_ms; /* the sort's kernels' time from CUDA events, or -1 when timing is off */
 } gqs_stats;
 
@@ -167,8 +170,8 @@ gqs_status gqs_sort_u32_noalloc(uint32_t* d, size_t n, void* stream);
  * (GPU-Quicksort_Full_SYCL/QuicksortMain.cpp:835-906); this is the batched form of that path. */
 typedef struct gqs_batch gqs_batch;
 
-/* cfg may be NULL; cfg->variant (>= 0) picks the initial kernel variant, cfg->timeout_ms the
- * device-side no-progress limit. */
+/* cfg may be NULL; cfg->variant (>= 0) picks the initial kernel variant (below 2^31 keys, of what
+ * the split leaves over), cfg->timeout_ms the device-side no-progress limit. */
 gqs_status gqs_batch_create(int device, int dtype, size_t max_keys, size_t max_segments, const gqs_config* cfg,
                             gqs_batch** out);
 void gqs_batch_destroy(gqs_batch* b);
@@ -189,7 +192,9 @@ gqs_status gqs_batch_copy_in(gqs_batch* b, const void* host, size_t first, size_
 gqs_status gqs_batch_copy_out(gqs_batch* b, void* host, size_t first, size_t n);
 gqs_status gqs_batch_set_variant(gqs_batch* b, int variant);
 int gqs_batch_get_variant(gqs_batch* b);
-/* The autotuner. Times every kernel variant of the batch's key type on the batch as it stands
+/* The autotuner. A batch of at least 2^31 keys is sorted by the variant alone; in a smaller one it
+ * only sorts what the split leaves over, seldom anything, and the variants then differ by less
+ * than the replays of one. Times every kernel variant of the batch's key type on the batch as it stands
  * (the first nseg segments of the table, keys restored from a copy before every replay): one
  * warm-up replay, then `reps` timed replays, median kept. Variants differ in the partition ->
  * on-chip sort switch (tile keys), CTA size (consumer warps) and keys per thread of a partition
@@ -220,7 +225,8 @@ typedef struct gqs_server_config {
   uint32_t timeout_ms;     /* device-side no-progress limit; 0 = 4000 */
   uint32_t per_request;    /* 1: no batching. One request at a time through the plain sort (copy
                               in, gqs_sort_<type>_dev, copy out, wait): the comparison baseline */
-  int32_t variant[3];      /* kernel variant per key type (GQS_U32, GQS_F32, GQS_F64); -1 = 0 */
+  int32_t variant[3];      /* kernel variant per key type (GQS_U32, GQS_F32, GQS_F64); -1 = 0 (with
+                              per_request: -1 = per sort, as in a context) */
   uint32_t reserved[4];
 } gqs_server_config;
 
@@ -293,7 +299,7 @@ gqs_status gqs_last_stats(gqs_ctx* ctx, gqs_stats* out);
  * (zeros otherwise). Writes up to n values and returns the number written. */
 int gqs_last_profile(gqs_ctx* ctx, uint64_t* out, size_t n);
 
-/* Where the last sort's persistent kernel spent its time, on the clock of each CTA's consumer
+/* Where the last sort's persistent kernel spent its time (zero if the split left it nothing), on the clock of each CTA's consumer
  * leader thread (SM cycles, summed over CTAs): on-chip sorts of ranges of at most one tile (the
  * lqsort_kernel counterpart: tile wait, sort, write-out), writes of queued pivot runs, and the
  * whole consumer loop; partition_cycles is the rest of the loop: partition chunk iterations (the
@@ -328,13 +334,14 @@ typedef struct gqs_level {
  * (libgqs_prof.so) records them; the product library returns 0. */
 int gqs_last_levels(gqs_ctx* ctx, gqs_level* out, int max);
 
-/* Kernel variants available for a key type (gqs_variant_describe: tile, chunk, CTA size). A
- * context created with cfg.variant = -1 picks, for every sort, the variant a tuning run on the
+/* Variants of the persistent kernel for a key type (gqs_variant_describe: tile, chunk, CTA size).
+ * It sorts what the split leaves over, arrays of 2^31 keys and more, and, in a context with a
+ * fixed variant, plain arrays of fewer than 2^15 or more than 2^21 keys by itself. A context created with cfg.variant = -1 picks, for every sort, the variant a tuning run on the
  * GPU found fastest for that key type and size class (ceil(log2 n)) on a GPU with the nearest
  * SM count: the counterpart of the reference's size-dependent launch parameters (optp,
  * GPU-Quicksort_Full_SYCL/QuicksortMain.cpp:831-833). gqs_set_variant fixes one variant for a key
- * type instead; gqs_get_variant returns it, or -1 while the context picks per sort (the variant a
- * sort ran with is in gqs_stats.variant). */
+ * type instead; gqs_get_variant returns it, or -1 while the context picks per sort (the variant
+ * chosen for a sort is in gqs_stats.variant). */
 int gqs_variant_count(int dtype);
 gqs_status gqs_variant_describe(int dtype, int variant, gqs_variant_desc* out);
 gqs_status gqs_set_variant(gqs_ctx* ctx, int dtype, int variant);
