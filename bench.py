@@ -17,7 +17,8 @@ uniformly over [0, 2^32) from a fixed seed. A step is one sort of that array.
             tests/golden/full_size.json: 2^20 u32; 2^28 u32 sorted / reverse / 16 distinct /
             Zipf(1.1) / Gaussian; 2^27 f32 N(0, 1e3); 2^26 f64 U[-1e9, 1e9]; the batched sort of
             4096 arrays (autotuned variant, against one plain call per array, end to end)
-  phases    the split of the 2^28 kernel's time between partition chunks and on-chip sorts
+  phases    the split of the persistent kernel's time between partition chunks and on-chip sorts (zero where
+            the sampled split has left it nothing)
 
 Options: --impl reference times the reference's CPU path (the oracle's restatement of
 GPUQSort<T>, all host threads) on the same 2^28 array, beside std::sort on one core and the
@@ -725,7 +726,7 @@ def run_batched(args, gqs_ctypes, rank, local, world, dist, barrier, clocks=None
            "api": "gqs_batch_copy_in + gqs_batch_launch + gqs_batch_wait + gqs_batch_copy_out (pinned)",
            "check": golden_check(case, hv, ov)}
     # the same arrays sorted by one plain call each (device pointers, enqueued back to back)
-    ctx = gqs_ctypes.Context(device=local, sync=False, timing=False, variant=0)
+    ctx = gqs_ctypes.Context(device=local, sync=False, timing=False)
     d = pristine.clone()
     dn = torch.empty_like(d)
     ctx.reserve("u32", int(np.diff(off).max()), 1)
@@ -758,7 +759,7 @@ def run_batched(args, gqs_ctypes, rank, local, world, dist, barrier, clocks=None
         "data": "synthetic (seeded generator, gpu-quicksort_gb300/workload)",
         "config": {"workload": workload_name(args, n, batched=True), "keys": n, "segments": nseg, "seed": SEED,
                    "l2": "inputs larger than L2 (arena rewritten from a pristine copy before every step)",
-                   "variant": chosen,
+                   "leftover_variant": chosen,
                    "graph": "one cudaGraphLaunch per step", "parallelism": f"replicas x{world}"},
         "autotune": tune,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
@@ -767,7 +768,7 @@ def run_batched(args, gqs_ctypes, rank, local, world, dist, barrier, clocks=None
         "kernel_ms": km,
         "plain_per_array": {"gkeys_s": n / (plain_ms / 1e3) / 1e9, "ms": plain_ms, "calls": nseg,
                             "same_output": plain_same, "batched_speedup": value / (n / (plain_ms / 1e3) / 1e9)},
-        "cpu_baseline": None, "e2e": e2e, "gpu_launches": 2 * steps, "clocks": clk, "check": check,
+        "cpu_baseline": None, "e2e": e2e, "gpu_launches": split_kernels(n, 4, segments=True) * steps, "clocks": clk, "check": check,
     }
 
 
@@ -835,12 +836,13 @@ def run_tiles(args, gqs_ctypes, rank, local, world, dist, barrier, peak, peak_sr
             "ms_per_step": 1e3 * t / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": args.dtype, "data": "synthetic (seeded generator, gpu-quicksort_gb300/workload)",
             "config": {"workload": workload_name(args, n), "keys": n, "segments": nseg, "segment_keys": seg,
-                       "variant": gqs_ctypes.variants(args.dtype)[st["variant"]]["name"]},
+                       "leftover_variant": gqs_ctypes.variants(args.dtype)[st["variant"]]["name"]},
             "roofline": {"bound": "hbm", "achieved": ab / (km / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": ab / (km / 1e3) / 1e9 / peak, "kernel_ms": km, "algo_bytes_per_launch": ab,
                          "peak_source": peak_src},
             "kernel_gkeys_s": n / (km / 1e3) / 1e9, "phases": phases, "clocks": clk,
-            "check": {"sampled_segments_equal_numpy_sort": bool(ok)}, "gpu_launches": 2 * args.steps}
+            "check": {"sampled_segments_equal_numpy_sort": bool(ok)},
+            "gpu_launches": split_kernels(n, esize, segments=True) * args.steps}
 
 
 class PlainRunner:
@@ -948,8 +950,13 @@ class PlainRunner:
                        if flush is None else "L2 flushed before every step (256 MiB write)")}
 
 
-def split_kernels(n, esize):
-    """Kernels of one plain sort of n keys (csrc/gqs_split.cu; the persistent kernel that may follow is not counted)."""
+def split_kernels(n, esize, segments=False, variant=-1):
+    """Kernels of one sort of n keys, or of segments with n keys in all (csrc/gqs_split.cu). The seed and persistent kernels
+    that follow for what may be left are not counted; they are counted where they sort alone."""
+    if n >= 1 << 31 or (variant >= 0 and not segments and not 1 << 15 <= n <= 1 << 21):
+        return 2
+    if segments:  # a plan in front, and two levels where the longest segment that n allows needs them
+        return 10 if n > 1024 * (3584 if esize == 4 else 1792) else 6
     if n <= (8192 if esize == 4 else 4096):
         return 1
     if n <= (1 << 21 if esize == 4 else 1 << 19):
@@ -962,7 +969,8 @@ def roofline_of(r, peak, peak_src, traffic=None):
     ab = float(np.mean(r["algo_bytes"]))
     achieved = ab / (km / 1e3) / 1e9
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": traffic, "kernel": "gqs split: map, count, starts, scatter (two levels), local_sort", "kernel_ms": km, "algo_bytes_per_launch": ab,
+            "traffic": traffic, "traffic_source": ncu_traffic("_about") if traffic else None,
+            "kernel": "gqs split: map, count, starts, scatter (two levels), local_sort", "kernel_ms": km, "algo_bytes_per_launch": ab,
             "peak_source": peak_src,
             "per_unit": f"{r['esize']} B x 2 per key per pass (partition chunks + on-chip sort + register sort)"}
 
@@ -995,7 +1003,7 @@ def run_configs(args, runner, clocks, peak, peak_src):
                     "roofline": {"achieved": rf["achieved"], "frac": rf["frac"], "peak": peak,
                                  "algo_bytes_per_launch": rf["algo_bytes_per_launch"]},
                     "passes_per_key": (st["part_keys"] + st["local_keys"] + st["tiny_keys"]) / r["n"],
-                    "variant": v["name"], "check": r["check"], "clocks": r["clocks"], "l2": r["l2"]})
+                    "leftover_variant": v["name"], "check": r["check"], "clocks": r["clocks"], "l2": r["l2"]})
     return out
 
 
@@ -1144,12 +1152,12 @@ def main():
         "ms_per_step": 1e3 * t_sort / args.steps, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": args.dtype, "data": "synthetic (seeded generator, gpu-quicksort_gb300/workload)",
         "config": {"workload": workload_name(args, n), "keys": n, "distribution": args.dist, "seed": SEED,
-                   "l2": r["l2"], "variant": v0["name"], "grid": stats_last["grid"],
-                   "threads": stats_last["threads"], "parallelism": f"replicas x{world}"},
+                   "l2": r["l2"], "kernel": v0["name"] if phases["total_cycles"] else "split",
+                   "leftover_variant": v0["name"], "parallelism": f"replicas x{world}"},
         "roofline": roofline,
         "cpu_baseline": cpu,
         "e2e": e2e,
-        "gpu_launches": split_kernels(n, r["esize"]) * args.steps,
+        "gpu_launches": split_kernels(n, r["esize"], variant=args.variant) * args.steps,
         "clocks": clk,
         "check": r["check"],
         "stats": {k: stats_last[k] for k in ("part_keys", "local_keys", "tiny_keys", "fill_keys", "chunks",
