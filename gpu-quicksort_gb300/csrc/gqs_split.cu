@@ -89,10 +89,10 @@ constexpr uint32_t kEqual = 1u << 30, kBinMask = 0xffffu;  // in a map's table: 
 struct SegRec {
   unsigned long long start;
   unsigned long long lo, span;  // keys are clamped to [lo, lo + span]
-  uint32_t len, k, cells;       // cells allocated (a power of two)
+  uint32_t len, k, cells;       // cells allocated, of the segment and of its parts
   uint32_t bin0, cell0, tile0;  // its counters, map cells and tiles
   uint32_t sh, bins, used;      // entries of the table; cell of a key: (key - lo) >> sh, or by value:
-  float flo, scale;             // (key - flo) * scale, in 4096ths of a cell
+  float flo, scale;             // (key - flo) * scale
   uint32_t top;                 // greatest value of that
   uint32_t kind;                // BY_VALUE, PARTS, and how many Part records there are
 };
